@@ -12,6 +12,7 @@
 //   Corner order LL, LR, RL, RR as set by solver_magnetic_utils (:32-49).
 #pragma once
 #include "dg_common.cuh"
+#include "round64.cuh"
 
 namespace dg {
 
@@ -30,17 +31,6 @@ template <typename T>
 __device__ __forceinline__ T cfast(T gamma, T ploc, T rho, T a, T b, T c) {
     return sqr(cfast2(gamma, ploc, rho, a, b, c));
 }
-// the same from b2 = a^2 + b^2 + c^2 computed by the caller: the x and y speeds of an edge
-// corner sum the same three squares in two orders, (A^2 + B^2) + C^2 and (B^2 + A^2) + C^2,
-// which are equal (IEEE addition commutes), so one b2 / rho serves both
-template <typename T>
-__device__ __forceinline__ T cfast2_b2(T gamma, T ploc, T rho, T a, T b2) {
-    const T half = T(0.5);
-    T c2 = gamma * ploc / rho;
-    T d2 = half * (c2 + b2 / rho);
-    return d2 + sqr(d2 * d2 - c2 * a * a / rho);
-}
-
 // left/right physical fluxes and conserved states shared by llf, hll, upwind
 template <typename T>
 __device__ __forceinline__ void lr_fluxes(const T *ql, const T *qr, T gamma, T ciso, int iso,
@@ -233,14 +223,13 @@ __device__ __forceinline__ void hlld1d_f(const float *ql, const float *qr, float
     pg = ptoto;
 }
 
-// HLLD; returns p*_T in pg.  entho = 1 / (gamma - 1), the same for every interface of a run
-// (formed once per context by the caller; the FP32 form takes its own reciprocal)
-template <typename T>
-__device__ void hlld1d(const T *ql, const T *qr, T *f, T &pg, T gamma, T ciso, int iso, T entho) {
-    if constexpr (sizeof(T) == 4) {
-        hlld1d_f(ql, qr, f, pg, gamma, ciso, iso);
-        return;
-    }
+// HLLD in FP64; returns p*_T in pg.  entho = 1 / (gamma - 1), the same for every interface of a run
+// (formed once per context by the caller).  M: IeeeMath, or FastMath whose caller tests m.bad().
+// Quotients by the negative sl - ustar are taken as (-numerator) / (ustar - sl), the same number.
+template <class M>
+__device__ __forceinline__ void hlld1d64(const double *ql, const double *qr, double *f, double &pg, double gamma,
+                                         double ciso, int iso, double entho, M &m) {
+    using T = double;
     const T half = T(0.5), zero = T(0);
     const T rl = ql[0], ul = ql[2], vl = ql[4], bl = ql[5], wl = ql[6], cl = ql[7];
     const T rr = qr[0], ur = qr[2], vr = qr[4], br = qr[5], wr = qr[6], cr = qr[7];
@@ -250,63 +239,80 @@ __device__ void hlld1d(const T *ql, const T *qr, T *f, T &pg, T gamma, T ciso, i
     if (iso) { ploc = rl * (ciso * ciso); proc = rr * (ciso * ciso); }
     else { ploc = ql[1]; proc = qr[1]; }
     const T ecinl = half * (ul * ul + vl * vl + wl * wl) * rl;
-    const T emagl = half * (a * a + bl * bl + cl * cl);
+    const T bsql = a * a + bl * bl + cl * cl;
+    const T emagl = half * bsql;
     const T etotl = ploc * entho + ecinl + emagl;
     const T ptotl = ploc + emagl;
     const T vdotbl = ul * a + vl * bl + wl * cl;
     const T ecinr = half * (ur * ur + vr * vr + wr * wr) * rr;
-    const T emagr = half * (a * a + br * br + cr * cr);
+    const T bsqr = a * a + br * br + cr * cr;
+    const T emagr = half * bsqr;
     const T etotr = proc * entho + ecinr + emagr;
     const T ptotr = proc + emagr;
     const T vdotbr = ur * a + vr * br + wr * cr;
-    const T cfmax = sqr(mx(cfast2(gamma, ploc, rl, a, bl, cl), cfast2(gamma, proc, rr, a, br, cr)));
+    // the fast speeds (cfast2 of each side), one root of the larger
+    const auto irl = m.rec(rl), irr = m.rec(rr);
+    const T c2l = m.div(gamma * ploc, rl, irl), c2r = m.div(gamma * proc, rr, irr);
+    const T d2l = half * (c2l + m.div(bsql, rl, irl)), d2r = half * (c2r + m.div(bsqr, rr, irr));
+    const T f2l = d2l + m.root(d2l * d2l - m.div(c2l * a * a, rl, irl));
+    const T f2r = d2r + m.root(d2r * d2r - m.div(c2r * a * a, rr, irr));
+    const T cfmax = m.root(mx(f2l, f2r));
     const T sl = mn(ul, ur) - cfmax;
     const T sr = mx(ul, ur) + cfmax;
     const T rcl = rl * (ul - sl);
     const T rcr = rr * (sr - ur);
-    const T ustar = (rcr * ur + rcl * ul + (ptotl - ptotr)) / (rcr + rcl);
-    const T ptotstar = (rcr * ptotl + rcl * ptotr + rcl * rcr * (ul - ur)) / (rcr + rcl);
+    const T rcs = rcr + rcl;
+    const auto ircs = m.rec(rcs);
+    const T ustar = m.div(rcr * ur + rcl * ul + (ptotl - ptotr), rcs, ircs);
+    const T ptotstar = m.div(rcr * ptotl + rcl * ptotr + rcl * rcr * (ul - ur), rcs, ircs);
     // left star region
-    const T rstarl = rl * (sl - ul) / (sl - ustar);
-    T estar = rl * (sl - ul) * (sl - ustar) - a * a;
+    const T usl = ustar - sl;
+    const auto iusl = m.rec(usl);
+    const T rstarl = m.div(-(rl * (sl - ul)), usl, iusl);
+    const T estarl = rl * (sl - ul) * (sl - ustar) - a * a;
     const T el = rl * (sl - ul) * (sl - ul) - a * a;
     T vstarl, bstarl, wstarl, cstarl;
-    if (estar == zero) { vstarl = vl; bstarl = bl; wstarl = wl; cstarl = cl; }
+    if (M::kZeroTest && estarl == zero) { vstarl = vl; bstarl = bl; wstarl = wl; cstarl = cl; }
     else {
-        vstarl = vl - a * bl * (ustar - ul) / estar;
-        bstarl = bl * el / estar;
-        wstarl = wl - a * cl * (ustar - ul) / estar;
-        cstarl = cl * el / estar;
+        const auto ie = m.rec(estarl);
+        vstarl = vl - m.div(a * bl * (ustar - ul), estarl, ie);
+        bstarl = m.div(bl * el, estarl, ie);
+        wstarl = wl - m.div(a * cl * (ustar - ul), estarl, ie);
+        cstarl = m.div(cl * el, estarl, ie);
     }
     const T vdotbstarl = ustar * a + vstarl * bstarl + wstarl * cstarl;
-    const T etotstarl = ((sl - ul) * etotl - ptotl * ul + ptotstar * ustar + a * (vdotbl - vdotbstarl)) / (sl - ustar);
-    const T sqrrstarl = sqr(rstarl);
-    const T calfvenl = fab(a) / sqrrstarl;
+    const T etotstarl = m.div(-((sl - ul) * etotl - ptotl * ul + ptotstar * ustar + a * (vdotbl - vdotbstarl)), usl, iusl);
+    typename M::Rec isql, isqr;
+    const T sqrrstarl = m.root(rstarl, isql);
+    const T calfvenl = m.div(fab(a), sqrrstarl, isql);
     const T sal = ustar - calfvenl;
     // right star region
-    const T rstarr = rr * (sr - ur) / (sr - ustar);
-    estar = rr * (sr - ur) * (sr - ustar) - a * a;
+    const T sru = sr - ustar;
+    const auto isru = m.rec(sru);
+    const T rstarr = m.div(rr * (sr - ur), sru, isru);
+    const T estarr = rr * (sr - ur) * (sr - ustar) - a * a;
     const T er = rr * (sr - ur) * (sr - ur) - a * a;
     T vstarr, bstarr, wstarr, cstarr;
-    if (estar == zero) { vstarr = vr; bstarr = br; wstarr = wr; cstarr = cr; }
+    if (M::kZeroTest && estarr == zero) { vstarr = vr; bstarr = br; wstarr = wr; cstarr = cr; }
     else {
-        vstarr = vr - a * br * (ustar - ur) / estar;
-        bstarr = br * er / estar;
-        wstarr = wr - a * cr * (ustar - ur) / estar;
-        cstarr = cr * er / estar;
+        const auto ie = m.rec(estarr);
+        vstarr = vr - m.div(a * br * (ustar - ur), estarr, ie);
+        bstarr = m.div(br * er, estarr, ie);
+        wstarr = wr - m.div(a * cr * (ustar - ur), estarr, ie);
+        cstarr = m.div(cr * er, estarr, ie);
     }
     const T vdotbstarr = ustar * a + vstarr * bstarr + wstarr * cstarr;
-    const T etotstarr = ((sr - ur) * etotr - ptotr * ur + ptotstar * ustar + a * (vdotbr - vdotbstarr)) / (sr - ustar);
-    const T sqrrstarr = sqr(rstarr);
-    const T calfvenr = fab(a) / sqrrstarr;
+    const T etotstarr = m.div((sr - ur) * etotr - ptotr * ur + ptotstar * ustar + a * (vdotbr - vdotbstarr), sru, isru);
+    const T sqrrstarr = m.root(rstarr, isqr);
+    const T calfvenr = m.div(fab(a), sqrrstarr, isqr);
     const T sar = ustar + calfvenr;
     // double star region
-    const T vstarstar = (sqrrstarl * vstarl + sqrrstarr * vstarr + sgnm * (bstarr - bstarl)) / (sqrrstarl + sqrrstarr);
-    const T wstarstar = (sqrrstarl * wstarl + sqrrstarr * wstarr + sgnm * (cstarr - cstarl)) / (sqrrstarl + sqrrstarr);
-    const T bstarstar = (sqrrstarl * bstarr + sqrrstarr * bstarl + sgnm * sqrrstarl * sqrrstarr * (vstarr - vstarl))
-                      / (sqrrstarl + sqrrstarr);
-    const T cstarstar = (sqrrstarl * cstarr + sqrrstarr * cstarl + sgnm * sqrrstarl * sqrrstarr * (wstarr - wstarl))
-                      / (sqrrstarl + sqrrstarr);
+    const T sqs = sqrrstarl + sqrrstarr;
+    const auto isqs = m.rec(sqs);
+    const T vstarstar = m.div(sqrrstarl * vstarl + sqrrstarr * vstarr + sgnm * (bstarr - bstarl), sqs, isqs);
+    const T wstarstar = m.div(sqrrstarl * wstarl + sqrrstarr * wstarr + sgnm * (cstarr - cstarl), sqs, isqs);
+    const T bstarstar = m.div(sqrrstarl * bstarr + sqrrstarr * bstarl + sgnm * sqrrstarl * sqrrstarr * (vstarr - vstarl), sqs, isqs);
+    const T cstarstar = m.div(sqrrstarl * cstarr + sqrrstarr * cstarl + sgnm * sqrrstarl * sqrrstarr * (wstarr - wstarl), sqs, isqs);
     const T vdotbstarstar = ustar * a + vstarstar * bstarstar + wstarstar * cstarstar;
     const T etotstarstarl = etotstarl - sgnm * sqrrstarl * (vdotbstarl - vdotbstarstar);
     const T etotstarstarr = etotstarr + sgnm * sqrrstarr * (vdotbstarr - vdotbstarstar);
@@ -338,6 +344,17 @@ __device__ void hlld1d(const T *ql, const T *qr, T *f, T &pg, T gamma, T ciso, i
     f[6] = ro * uo * wo - a * co;
     f[7] = co * uo - a * wo;
     pg = ptoto;
+}
+
+// HLLD, either arithmetic
+template <typename T>
+__device__ void hlld1d(const T *ql, const T *qr, T *f, T &pg, T gamma, T ciso, int iso, T entho) {
+    if constexpr (sizeof(T) == 4) {
+        hlld1d_f(ql, qr, f, pg, gamma, ciso, iso);
+    } else {
+        IeeeMath m;
+        hlld1d64(ql, qr, f, pg, gamma, ciso, iso, entho, m);
+    }
 }
 
 // the four corner states of an edge after solver_magnetic_utils
@@ -460,34 +477,47 @@ __device__ __forceinline__ float hlld2d_f(const Corners<float> &c, float dt, flo
     return E * dt;
 }
 
-template <typename T>
-__device__ T hlld2d(const Corners<T> &c, T dt, T gamma) {
-    if constexpr (sizeof(T) == 4) return hlld2d_f(c, dt, gamma);
-    const T one = T(1), half = T(0.5), zero = T(0), smallc = T(kSmallc);
+// 2D HLLD in FP64 (M as in hlld1d64); reciprocals of the negative SL - ustar and SB - vstar are
+// taken as -1 / (ustar - SL) and -1 / (vstar - SB)
+template <class M>
+__device__ __forceinline__ double hlld2d64(const Corners<double> &c, double dt, double gamma, M &m) {
+    using T = double;
+    const T half = T(0.5), zero = T(0), smallc = T(kSmallc);
     const T b2LL = c.ALL * c.ALL + c.BLL * c.BLL + c.CLL * c.CLL, b2LR = c.ALR * c.ALR + c.BLR * c.BLR + c.CLR * c.CLR;
     const T b2RL = c.ARL * c.ARL + c.BRL * c.BRL + c.CRL * c.CRL, b2RR = c.ARR * c.ARR + c.BRR * c.BRR + c.CRR * c.CRR;
-    const T cfx = sqr(mx4(cfast2_b2(gamma, c.pLL, c.rLL, c.ALL, b2LL), cfast2_b2(gamma, c.pLR, c.rLR, c.ALR, b2LR),
-                          cfast2_b2(gamma, c.pRL, c.rRL, c.ARL, b2RL), cfast2_b2(gamma, c.pRR, c.rRR, c.ARR, b2RR)));
-    const T cfy = sqr(mx4(cfast2_b2(gamma, c.pLL, c.rLL, c.BLL, b2LL), cfast2_b2(gamma, c.pLR, c.rLR, c.BLR, b2LR),
-                          cfast2_b2(gamma, c.pRL, c.rRL, c.BRL, b2RL), cfast2_b2(gamma, c.pRR, c.rRR, c.BRR, b2RR)));
+    // the squared fast speeds of a corner along x and y (cfast2): c2 = gamma p / rho, the sum of the
+    // squares in either order is the same number, so one quotient by rho serves both
+    auto fast = [&](T p, T r, T a, T b, T b2, T &fx, T &fy) {
+        const auto ir = m.rec(r);
+        const T c2 = m.div(gamma * p, r, ir);
+        const T d2 = half * (c2 + m.div(b2, r, ir));
+        fx = d2 + m.root(d2 * d2 - m.div(c2 * a * a, r, ir));
+        fy = d2 + m.root(d2 * d2 - m.div(c2 * b * b, r, ir));
+    };
+    T xLL, yLL, xLR, yLR, xRL, yRL, xRR, yRR;
+    fast(c.pLL, c.rLL, c.ALL, c.BLL, b2LL, xLL, yLL);
+    fast(c.pLR, c.rLR, c.ALR, c.BLR, b2LR, xLR, yLR);
+    fast(c.pRL, c.rRL, c.ARL, c.BRL, b2RL, xRL, yRL);
+    fast(c.pRR, c.rRR, c.ARR, c.BRR, b2RR, xRR, yRR);
+    const T cfx = m.root(mx4(xLL, xLR, xRL, xRR));
+    const T cfy = m.root(mx4(yLL, yLR, yRL, yRR));
     const T SL = mn4(c.uLL, c.uLR, c.uRL, c.uRR) - cfx;
     const T SR = mx4(c.uLL, c.uLR, c.uRL, c.uRR) + cfx;
     const T SB = mn4(c.vLL, c.vLR, c.vRL, c.vRR) - cfy;
     const T ST = mx4(c.vLL, c.vLR, c.vRL, c.vRR) + cfy;
-    const T PtotLL = c.pLL + half * (c.ALL * c.ALL + c.BLL * c.BLL + c.CLL * c.CLL);
-    const T PtotLR = c.pLR + half * (c.ALR * c.ALR + c.BLR * c.BLR + c.CLR * c.CLR);
-    const T PtotRL = c.pRL + half * (c.ARL * c.ARL + c.BRL * c.BRL + c.CRL * c.CRL);
-    const T PtotRR = c.pRR + half * (c.ARR * c.ARR + c.BRR * c.BRR + c.CRR * c.CRR);
+    const T PtotLL = c.pLL + half * b2LL, PtotLR = c.pLR + half * b2LR;
+    const T PtotRL = c.pRL + half * b2RL, PtotRR = c.pRR + half * b2RR;
     const T rcLLx = c.rLL * (c.uLL - SL), rcRLx = c.rRL * (SR - c.uRL);
     const T rcLRx = c.rLR * (c.uLR - SL), rcRRx = c.rRR * (SR - c.uRR);
     const T rcLLy = c.rLL * (c.vLL - SB), rcLRy = c.rLR * (ST - c.vLR);
     const T rcRLy = c.rRL * (c.vRL - SB), rcRRy = c.rRR * (ST - c.vRR);
-    const T ustar = (rcLLx * c.uLL + rcLRx * c.uLR + rcRLx * c.uRL + rcRRx * c.uRR + (PtotLL - PtotRL + PtotLR - PtotRR))
-                  / (rcLLx + rcLRx + rcRLx + rcRRx);
-    const T vstar = (rcLLy * c.vLL + rcLRy * c.vLR + rcRLy * c.vRL + rcRRy * c.vRR + (PtotLL - PtotLR + PtotRL - PtotRR))
-                  / (rcLLy + rcLRy + rcRLy + rcRRy);
-    const T SLustar = one / (SL - ustar), SRustar = one / (SR - ustar);
-    const T SBvstar = one / (SB - vstar), STvstar = one / (ST - vstar);
+    const T rcx = rcLLx + rcLRx + rcRLx + rcRRx, rcy = rcLLy + rcLRy + rcRLy + rcRRy;
+    const T ustar = m.div(rcLLx * c.uLL + rcLRx * c.uLR + rcRLx * c.uRL + rcRRx * c.uRR + (PtotLL - PtotRL + PtotLR - PtotRR),
+                          rcx, m.rec(rcx));
+    const T vstar = m.div(rcLLy * c.vLL + rcLRy * c.vLR + rcRLy * c.vRL + rcRRy * c.vRR + (PtotLL - PtotLR + PtotRL - PtotRR),
+                          rcy, m.rec(rcy));
+    const T SLustar = -m.inv(ustar - SL), SRustar = m.inv(SR - ustar);
+    const T SBvstar = -m.inv(vstar - SB), STvstar = m.inv(ST - vstar);
     const T rstarLLx = c.rLL * (SL - c.uLL) * SLustar;
     const T BstarLL = c.BLL * (SL - c.uLL) * SLustar;
     const T rstarLLy = c.rLL * (SB - c.vLL) * SBvstar;
@@ -520,22 +550,27 @@ __device__ T hlld2d(const Corners<T> &c, T dt, T gamma) {
     const T EstarRRx = ustar * BstarRR - c.vRR * c.ARR;
     const T EstarRRy = c.uRR * c.BRR - vstar * AstarRR;
     const T EstarRR = ustar * BstarRR - vstar * AstarRR;
-    const T sqrtrstarLR = one / sqr(rstarLR);
-    const T sqrtrstarRL = one / sqr(rstarRL);
-    const T sqrtrstarRR = one / sqr(rstarRR);
-    const T sqrtrstarLL = one / sqr(rstarLL);
-    const T calfvenL = mx(mx(mx(mx(fab(c.ALR) / sqr(rstarLRx), fab(AstarLR) * sqrtrstarLR),
-                                fab(c.ALL) / sqr(rstarLLx)), fab(AstarLL) * sqrtrstarLL), smallc);
-    const T calfvenR = mx(mx(mx(mx(fab(c.ARR) / sqr(rstarRRx), fab(AstarRR) * sqrtrstarRR),
-                                fab(c.ARL) / sqr(rstarRLx)), fab(AstarRL) * sqrtrstarRL), smallc);
-    const T calfvenB = mx(mx(mx(mx(fab(c.BLL) / sqr(rstarLLy), fab(BstarLL) * sqrtrstarLL),
-                                fab(c.BRL) / sqr(rstarRLy)), fab(BstarRL) * sqrtrstarRL), smallc);
-    const T calfvenT = mx(mx(mx(mx(fab(c.BLR) / sqr(rstarLRy), fab(BstarLR) * sqrtrstarLR),
-                                fab(c.BRR) / sqr(rstarRRy)), fab(BstarRR) * sqrtrstarRR), smallc);
+    const T sqrtrstarLR = m.inv_root(rstarLR);
+    const T sqrtrstarRL = m.inv_root(rstarRL);
+    const T sqrtrstarRR = m.inv_root(rstarRR);
+    const T sqrtrstarLL = m.inv_root(rstarLL);
+    auto per_root = [&](T a, T r) {  // |a| / sqrt(r)
+        typename M::Rec z;
+        const T s = m.root(r, z);
+        return m.div(fab(a), s, z);
+    };
+    const T calfvenL = mx(mx(mx(mx(per_root(c.ALR, rstarLRx), fab(AstarLR) * sqrtrstarLR),
+                                per_root(c.ALL, rstarLLx)), fab(AstarLL) * sqrtrstarLL), smallc);
+    const T calfvenR = mx(mx(mx(mx(per_root(c.ARR, rstarRRx), fab(AstarRR) * sqrtrstarRR),
+                                per_root(c.ARL, rstarRLx)), fab(AstarRL) * sqrtrstarRL), smallc);
+    const T calfvenB = mx(mx(mx(mx(per_root(c.BLL, rstarLLy), fab(BstarLL) * sqrtrstarLL),
+                                per_root(c.BRL, rstarRLy)), fab(BstarRL) * sqrtrstarRL), smallc);
+    const T calfvenT = mx(mx(mx(mx(per_root(c.BLR, rstarLRy), fab(BstarLR) * sqrtrstarLR),
+                                per_root(c.BRR, rstarRRy)), fab(BstarRR) * sqrtrstarRR), smallc);
     const T SAL = mn(ustar - calfvenL, zero), SAR = mx(ustar + calfvenR, zero);
     const T SAB = mn(vstar - calfvenB, zero), SAT = mx(vstar + calfvenT, zero);
-    const T SARSAL = one / (SAR - SAL);
-    const T SATSAB = one / (SAT - SAB);
+    const T SARSAL = m.inv(SAR - SAL);
+    const T SATSAB = m.inv(SAT - SAB);
     const T AstarT = (SAR * AstarRR - SAL * AstarLR) * SARSAL;
     const T AstarB = (SAR * AstarRL - SAL * AstarLL) * SARSAL;
     const T BstarR = (SAT * BstarRR - SAB * BstarRL) * SATSAB;
@@ -558,6 +593,16 @@ __device__ T hlld2d(const Corners<T> &c, T dt, T gamma) {
           - SAT * SAB * SATSAB * (AstarT - AstarB) + SAR * SAL * SARSAL * (BstarR - BstarL);
     }
     return E * dt;
+}
+
+template <typename T>
+__device__ T hlld2d(const Corners<T> &c, T dt, T gamma) {
+    if constexpr (sizeof(T) == 4) {
+        return hlld2d_f(c, dt, gamma);
+    } else {
+        IeeeMath m;
+        return hlld2d64(c, dt, gamma, m);
+    }
 }
 
 template <typename T>

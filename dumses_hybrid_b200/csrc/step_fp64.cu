@@ -251,6 +251,54 @@ __global__ void __launch_bounds__(kThreads) k_update2d(Geo G, const double *__re
 }
 
 
+// HLLD/HLLD: the six kinds of solve (faces x, y, z, edges x, y, z) as one grid.  Bound by the FP64
+// pipe (54% of its cycles at 128^3) and the latency in front of it: the core's loads and dependent
+// FP64 instructions.  A block does one kind for 128 points of the face index space; the grid runs
+// the kinds one after the other over chunks of DG_RIEMANN_CHUNK64 tiles, so that an SM's blocks
+// mostly share one kind's code (a sixth of the whole) while the chunk's trace core, read from HBM by
+// the first kind, is in L2 for the others: 0.88 GB of HBM reads at 128^3 against 2.0 GB for a kernel
+// per kind.  At 256^3 (MRI, FARGO): six kernels with IEEE operators 7.21 ms, with round64.cuh 5.96,
+// this grid 5.69 (chunks of 148 tiles 6.65, 370 5.83, 1480 5.75, 2960 5.79; 4 blocks per SM instead
+// of 5: 5.87; 6 blocks, as six kernels: 7.20 with spills); at 64^3 0.184 -> 0.110 ms, where a kernel
+// per kind is less than one wave.
+#ifndef DG_RIEMANN_CHUNK64
+#define DG_RIEMANN_CHUNK64 740
+#endif
+#ifndef DG_RIEMANN_ALL_MINB64
+#define DG_RIEMANN_ALL_MINB64 5
+#endif
+struct RiemannGrid {
+    unsigned chunk, blocks;  // tiles per chunk (equal chunks: a few spare blocks of the last one return at once)
+};
+inline RiemannGrid riemann64_grid(const Geo &G) {
+    const unsigned tiles = nblocks(G.fsz, kThreads);
+    const unsigned n = (tiles + DG_RIEMANN_CHUNK64 - 1) / DG_RIEMANN_CHUNK64, chunk = (tiles + n - 1) / n;
+    return RiemannGrid{chunk, 6 * n * chunk};
+}
+__global__ void __launch_bounds__(kThreads, DG_RIEMANN_ALL_MINB64)
+k_riemann64(const __grid_constant__ Geo G, unsigned nc, const double *__restrict__ core, double *__restrict__ fx,
+            double *__restrict__ fy, double *__restrict__ fz, double *__restrict__ ex, double *__restrict__ ey,
+            double *__restrict__ ez, const Scalars *S) {
+    const unsigned chunk = blockIdx.x / (6 * nc), r = blockIdx.x - chunk * (6 * nc);
+    const unsigned kind = r / nc, tile = chunk * nc + (r - kind * nc);
+    const long long t = tile * (long long)kThreads + threadIdx.x;
+    if (t >= G.fsz) return;
+    int i, j, k;
+    split3((unsigned)t, G.dFX, G.dFY, i, j, k);
+    i++; j++; k++;
+    const double dt = S->dt;
+    const long long c = G.cidx(i, j, k);
+    const long long px = 1, py = G.CX, pz = (long long)G.CX * G.CY;  // core index steps
+    switch (kind) {
+        case 0: if (j <= G.ny && k <= G.nz) face_flux_fast<0>(G, core, c - px, c, i, dt, fx, t); break;
+        case 1: if (i <= G.nx && k <= G.nz) face_flux_fast<1>(G, core, c - py, c, i, dt, fy, t); break;
+        case 2: if (i <= G.nx && j <= G.ny) face_flux_fast<2>(G, core, c - pz, c, i, dt, fz, t); break;
+        case 3: if (i <= G.nx) ex[t] = edge_emf_fast<0>(G, core, c - py - pz, c - pz, c - py, c, i, dt); break;
+        case 4: if (j <= G.ny) ey[t] = edge_emf_fast<1>(G, core, c - px - pz, c - px, c - pz, c, i, dt); break;
+        default: if (k <= G.nz) ez[t] = edge_emf_fast<2>(G, core, c - px - py, c - py, c - px, c, i, dt); break;
+    }
+}
+
 StoreD st(const Bufs &B, int b) { return StoreD{(double *)B.U[b]}; }
 
 }  // namespace
@@ -306,18 +354,6 @@ constexpr bool kTraceSplit64 = DG_TRACE_SPLIT64 != 0;
 #endif
 constexpr bool kTraceTile64 = DG_TRACE_TILE64 != 0;
 
-// 3D Riemann work as two kernels (faces, then edges) instead of one
-#ifndef DG_RIEMANN_SPLIT64
-#define DG_RIEMANN_SPLIT64 1
-#endif
-constexpr bool kRiemannSplit64 = DG_RIEMANN_SPLIT64 != 0;
-// HLLD/HLLD: one kernel per direction for the faces and for the edges (six launches; each
-// kernel's code is a third of the two-kernel form's, and 7.57 against 8.22 ms at 256^3)
-#ifndef DG_RIEMANN_PERDIR64
-#define DG_RIEMANN_PERDIR64 1
-#endif
-constexpr bool kRiemannPerDir64 = DG_RIEMANN_PERDIR64 != 0;
-
 int launch_godunov(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
     const StoreD U = st(B, cur);
     double *Un = (double *)B.U[cur ^ 1];
@@ -352,29 +388,16 @@ int launch_godunov(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
         } else {
             TIMED(KS_TRACE, s, (k_trace3d<double><<<nblocks(G.csz, kThreads), kThreads, 0, s>>>(G, Q, U.p, E0, E1, E2, core, B.S)));
         }
-        // HLLD/HLLD (the reference's default and every benchmark) runs kernels without the other solvers
+        // HLLD/HLLD (the reference's default and every benchmark) runs its own kernel, the other
+        // solvers one kernel for the faces and one for the edges
         const unsigned nb = nblocks(G.fsz, kThreads);
-        if (kRiemannPerDir64 && G.iriemann == DG_RIEMANN_HLLD && G.iriemann2d == DG_RIEMANN_HLLD) {
-            TIMED(KS_RIEMANN, s, (k_faces3d<double, true, 0><<<nb, kThreads, 0, s>>>(G, core, fx, fy, fz, B.S)));
-            TIMED(KS_RIEMANN, s, (k_faces3d<double, true, 1><<<nb, kThreads, 0, s>>>(G, core, fx, fy, fz, B.S)));
-            TIMED(KS_RIEMANN, s, (k_faces3d<double, true, 2><<<nb, kThreads, 0, s>>>(G, core, fx, fy, fz, B.S)));
-            TIMED(KS_RIEMANN, s, (k_edges3d<double, true, 0><<<nb, kThreads, 0, s>>>(G, core, ex, ey, ez, B.S)));
-            TIMED(KS_RIEMANN, s, (k_edges3d<double, true, 1><<<nb, kThreads, 0, s>>>(G, core, ex, ey, ez, B.S)));
-            TIMED(KS_RIEMANN, s, (k_edges3d<double, true, 2><<<nb, kThreads, 0, s>>>(G, core, ex, ey, ez, B.S)));
-            n += 5;
-        } else if (kRiemannSplit64) {
-            if (G.iriemann == DG_RIEMANN_HLLD && G.iriemann2d == DG_RIEMANN_HLLD) {
-                TIMED(KS_RIEMANN, s, (k_faces3d<double, true><<<nb, kThreads, 0, s>>>(G, core, fx, fy, fz, B.S)));
-                TIMED(KS_RIEMANN, s, (k_edges3d<double, true><<<nb, kThreads, 0, s>>>(G, core, ex, ey, ez, B.S)));
-            } else {
-                TIMED(KS_RIEMANN, s, (k_faces3d<double, false><<<nb, kThreads, 0, s>>>(G, core, fx, fy, fz, B.S)));
-                TIMED(KS_RIEMANN, s, (k_edges3d<double, false><<<nb, kThreads, 0, s>>>(G, core, ex, ey, ez, B.S)));
-            }
-            n++;
-        } else if (G.iriemann == DG_RIEMANN_HLLD && G.iriemann2d == DG_RIEMANN_HLLD) {
-            TIMED(KS_RIEMANN, s, (k_riemann3d<double, true><<<nb, kThreads, 0, s>>>(G, core, fx, fy, fz, ex, ey, ez, B.S, 1)));
+        if (G.iriemann == DG_RIEMANN_HLLD && G.iriemann2d == DG_RIEMANN_HLLD) {
+            const RiemannGrid rg = riemann64_grid(G);
+            TIMED(KS_RIEMANN, s, (k_riemann64<<<rg.blocks, kThreads, 0, s>>>(G, rg.chunk, core, fx, fy, fz, ex, ey, ez, B.S)));
         } else {
-            TIMED(KS_RIEMANN, s, (k_riemann3d<double, false><<<nb, kThreads, 0, s>>>(G, core, fx, fy, fz, ex, ey, ez, B.S, 1)));
+            TIMED(KS_RIEMANN, s, (k_faces3d<double, false><<<nb, kThreads, 0, s>>>(G, core, fx, fy, fz, B.S)));
+            TIMED(KS_RIEMANN, s, (k_edges3d<double, false><<<nb, kThreads, 0, s>>>(G, core, ex, ey, ez, B.S)));
+            n++;
         }
         TIMED(KS_UPDATE, s, (k_update3d<<<nblocks(G.fsz, kThreads), kThreads, 0, s>>>(G, U.p, Un, fx, fy, fz, ex, ey, ez, B.S)));
     } else if (G.ndim == 1) {

@@ -1268,10 +1268,10 @@ __device__ void face_flux(const Geo &G, const CoreView<T> &cv, long long cl, lon
     flux_store(G, ql, qr, f, pg, d, i, dtd, out, fo);
 }
 
-// one edge EMF (riemann_solver_magnetic, solver_magnetic.f90:79-230); e = edge direction
-template <typename T, bool kHLLD = false>
-__device__ T edge_emf(const Geo &G, const CoreView<T> &cv, long long cLL, long long cRL, long long cLR, long long cRR,
-                      int e, int i, double dtd) {
+// the four corner states of an edge (riemann_solver_magnetic, solver_magnetic.f90:79-180); e = edge direction
+template <typename T>
+__device__ __forceinline__ void edge_corners(const Geo &G, const CoreView<T> &cv, long long cLL, long long cRL,
+                                             long long cLR, long long cRR, int e, Corners<T> &c) {
     const T half = T(0.5);
     const T smallp = (T)G.smallp;
     T sLL[8], sRL[8], sLR[8], sRR[8];
@@ -1322,7 +1322,6 @@ __device__ T edge_emf(const Geo &G, const CoreView<T> &cv, long long cLL, long l
     qRL[7] = qRL[2] * qRL[5] - qRL[3] * qRL[4];
     qLR[7] = qLR[2] * qLR[5] - qLR[3] * qLR[4];
     qRR[7] = qRR[2] * qRR[5] - qRR[3] * qRR[4];
-    Corners<T> c;
     c.rLL = qLL[0]; c.uLL = qLL[2]; c.ALL = qLL[4]; c.CLL = qLL[6];
     c.rRL = qRL[0]; c.uRL = qRL[2]; c.ARL = qRL[4]; c.CRL = qRL[6];
     c.rLR = qLR[0]; c.uLR = qLR[2]; c.ALR = qLR[4]; c.CLR = qLR[6];
@@ -1331,15 +1330,11 @@ __device__ T edge_emf(const Geo &G, const CoreView<T> &cv, long long cLL, long l
     c.pRL = qRL[1]; c.vRL = qRL[3]; c.BRL = qRL[5]; c.ERL = qRL[7];
     c.pLR = qLR[1]; c.vLR = qLR[3]; c.BLR = qLR[5]; c.ELR = qLR[7];
     c.pRR = qRR[1]; c.vRR = qRR[3]; c.BRR = qRR[5]; c.ERR = qRR[7];
-    const T dt = (T)dtd, gamma = (T)G.gamma;
-    T emf;
-    if constexpr (kHLLD) emf = hlld2d<T>(c, dt, gamma);
-    else switch (G.iriemann2d) {
-        case DG_RIEMANN_HLLD: emf = hlld2d<T>(c, dt, gamma); break;
-        case DG_RIEMANN_LLF: emf = llf2d<T>(c, dt, gamma, (T)G.ciso, G.iso); break;
-        case DG_RIEMANN_HLLA: emf = hlla2d<T>(c, dt); break;
-        default: emf = upwind2d<T>(c, dt); break;
-    }
+}
+
+// the shearing-box upwind terms of an edge EMF (solver_magnetic.f90:181-230)
+template <typename T>
+__device__ __forceinline__ T edge_shear(const Geo &G, const Corners<T> &c, T emf, int e, int i, T dt) {
     if ((G.omega0 > 0.0) && !G.fargo) {
         if (e == 0) {
             const T shear = (T)(-1.5 * G.omega0 * G.xc(i));
@@ -1352,6 +1347,24 @@ __device__ T edge_emf(const Geo &G, const CoreView<T> &cv, long long cLL, long l
         }
     }
     return emf;
+}
+
+// one edge EMF (riemann_solver_magnetic, solver_magnetic.f90:79-230); e = edge direction
+template <typename T, bool kHLLD = false>
+__device__ T edge_emf(const Geo &G, const CoreView<T> &cv, long long cLL, long long cRL, long long cLR, long long cRR,
+                      int e, int i, double dtd) {
+    Corners<T> c;
+    edge_corners(G, cv, cLL, cRL, cLR, cRR, e, c);
+    const T dt = (T)dtd, gamma = (T)G.gamma;
+    T emf;
+    if constexpr (kHLLD) emf = hlld2d<T>(c, dt, gamma);
+    else switch (G.iriemann2d) {
+        case DG_RIEMANN_HLLD: emf = hlld2d<T>(c, dt, gamma); break;
+        case DG_RIEMANN_LLF: emf = llf2d<T>(c, dt, gamma, (T)G.ciso, G.iso); break;
+        case DG_RIEMANN_HLLA: emf = hlla2d<T>(c, dt); break;
+        default: emf = upwind2d<T>(c, dt); break;
+    }
+    return edge_shear(G, c, emf, e, i, dt);
 }
 
 template <typename T, bool kHLLD>
@@ -1381,6 +1394,48 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 ? DG_RIEMANN_MINB64 
         ex[t] = edge_emf<T, kHLLD>(G, cv, G.cidx(i, j - 1, k - 1), G.cidx(i, j, k - 1), G.cidx(i, j - 1, k), c, 0, i, dt);
 }
 
+// FP64 HLLD/HLLD solves of one direction with the straight-line arithmetic of round64.cuh; a solve
+// with an operand outside its range is done again by the *_ieee form (out of line: a kernel's
+// fast path carries only the call).  The kernels take Geo as a __grid_constant__, so that the
+// reference these calls pass needs no copy of it per thread.
+template <int kDir>
+__device__ __noinline__ void face_flux_ieee(const Geo &G, const double *core, long long cl, long long cr, int i,
+                                            double dtd, double *out, long long fo) {
+    const CoreView<double> cv{core, kCore3};
+    face_flux<double, true>(G, cv, cl, cr, kDir, i, dtd, out, fo);
+}
+template <int kDir>
+__device__ __forceinline__ void face_flux_fast(const Geo &G, const double *core, long long cl, long long cr, int i,
+                                               double dtd, double *__restrict__ out, long long fo) {
+    const CoreView<double> cv{core, kCore3};
+    double ql[8], qr[8], f[8], pg;
+    face_io(G, cv, cl, cr, kDir, ql, qr);
+    FastMath m;
+    hlld1d64(ql, qr, f, pg, G.gamma, G.ciso, G.iso, G.entho, m);
+    if (m.bad()) {
+        face_flux_ieee<kDir>(G, core, cl, cr, i, dtd, out, fo);
+        return;
+    }
+    flux_store(G, ql, qr, f, pg, kDir, i, dtd, out, fo);
+}
+template <int kDir>
+__device__ __noinline__ double edge_emf_ieee(const Geo &G, const double *core, long long cLL, long long cRL,
+                                             long long cLR, long long cRR, int i, double dtd) {
+    const CoreView<double> cv{core, kCore3};
+    return edge_emf<double, true>(G, cv, cLL, cRL, cLR, cRR, kDir, i, dtd);
+}
+template <int kDir>
+__device__ __forceinline__ double edge_emf_fast(const Geo &G, const double *core, long long cLL, long long cRL,
+                                                long long cLR, long long cRR, int i, double dtd) {
+    const CoreView<double> cv{core, kCore3};
+    Corners<double> c;
+    edge_corners(G, cv, cLL, cRL, cLR, cRR, kDir, c);
+    FastMath m;
+    const double emf = hlld2d64(c, dtd, G.gamma, m);
+    if (m.bad()) return edge_emf_ieee<kDir>(G, core, cLL, cRL, cLR, cRR, i, dtd);
+    return edge_shear(G, c, emf, kDir, i, dtd);
+}
+
 // The same work split in two passes over the face index space: the face fluxes (1D solves)
 // and the edge EMFs (2D solves), each compiled for its own register budget.  A thread
 // holds the live values of one kind of solve only, so more warps fit an SM; the trace core
@@ -1398,8 +1453,7 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 ? DG_RIEMANN_MINB64 
 #ifndef DG_REDGE_MINB32
 #define DG_REDGE_MINB32 8
 #endif
-// kDir: the one direction this launch solves (0, 1, 2), or -1 for all three
-template <typename T, bool kHLLD, int kDir = -1>
+template <typename T, bool kHLLD>
 __global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 ? DG_RFACE_MINB64 : DG_RFACE_MINB32))
 k_faces3d(Geo G, const T *__restrict__ core, T *__restrict__ fx, T *__restrict__ fy, T *__restrict__ fz,
           const Scalars *S) {
@@ -1411,12 +1465,12 @@ k_faces3d(Geo G, const T *__restrict__ core, T *__restrict__ fx, T *__restrict__
     const double dt = S->dt;
     const CoreView<T> cv{core, kCore3};
     const long long c = G.cidx(i, j, k);
-    if ((kDir < 0 || kDir == 0) && j <= G.ny && k <= G.nz) face_flux<T, kHLLD>(G, cv, G.cidx(i - 1, j, k), c, 0, i, dt, fx, t);
-    if ((kDir < 0 || kDir == 1) && i <= G.nx && k <= G.nz) face_flux<T, kHLLD>(G, cv, G.cidx(i, j - 1, k), c, 1, i, dt, fy, t);
-    if ((kDir < 0 || kDir == 2) && i <= G.nx && j <= G.ny) face_flux<T, kHLLD>(G, cv, G.cidx(i, j, k - 1), c, 2, i, dt, fz, t);
+    if (j <= G.ny && k <= G.nz) face_flux<T, kHLLD>(G, cv, G.cidx(i - 1, j, k), c, 0, i, dt, fx, t);
+    if (i <= G.nx && k <= G.nz) face_flux<T, kHLLD>(G, cv, G.cidx(i, j - 1, k), c, 1, i, dt, fy, t);
+    if (i <= G.nx && j <= G.ny) face_flux<T, kHLLD>(G, cv, G.cidx(i, j, k - 1), c, 2, i, dt, fz, t);
 }
 
-template <typename T, bool kHLLD, int kDir = -1>
+template <typename T, bool kHLLD>
 __global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 ? DG_REDGE_MINB64 : DG_REDGE_MINB32))
 k_edges3d(Geo G, const T *__restrict__ core, T *__restrict__ ex, T *__restrict__ ey, T *__restrict__ ez,
           const Scalars *S) {
@@ -1428,11 +1482,11 @@ k_edges3d(Geo G, const T *__restrict__ core, T *__restrict__ ex, T *__restrict__
     const double dt = S->dt;
     const CoreView<T> cv{core, kCore3};
     const long long c = G.cidx(i, j, k);
-    if ((kDir < 0 || kDir == 2) && k <= G.nz)
+    if (k <= G.nz)
         ez[t] = edge_emf<T, kHLLD>(G, cv, G.cidx(i - 1, j - 1, k), G.cidx(i, j - 1, k), G.cidx(i - 1, j, k), c, 2, i, dt);
-    if ((kDir < 0 || kDir == 1) && j <= G.ny)
+    if (j <= G.ny)
         ey[t] = edge_emf<T, kHLLD>(G, cv, G.cidx(i - 1, j, k - 1), G.cidx(i - 1, j, k), G.cidx(i, j, k - 1), c, 1, i, dt);
-    if ((kDir < 0 || kDir == 0) && i <= G.nx)
+    if (i <= G.nx)
         ex[t] = edge_emf<T, kHLLD>(G, cv, G.cidx(i, j - 1, k - 1), G.cidx(i, j, k - 1), G.cidx(i, j - 1, k), c, 0, i, dt);
 }
 
