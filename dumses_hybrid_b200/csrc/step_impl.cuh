@@ -640,12 +640,30 @@ __device__ __forceinline__ void trace3_cell(const Sten &a, const Geo &G, int i, 
 
     // source terms, scheme.f90:1351-1389
     T sr0 = (-u * drx - dux * r) * dtdx + (-v * dry - dvy * r) * dtdy + (-w * drz - dwz * r) * dtdz;
-    T su0 = (-u * dux - (dpx + B * dBx + C * dCx) / r) * dtdx + (-v * duy + B * dAy / r) * dtdy
-          + (-w * duz + C * dAz / r) * dtdz;
-    T sv0 = (-u * dvx + A * dBx / r) * dtdx + (-v * dvy - (dpy + A * dAy + C * dCy) / r) * dtdy
-          + (-w * dvz + C * dBz / r) * dtdz;
-    T sw0 = (-u * dwx + A * dCx / r) * dtdx + (-v * dwy + B * dCy / r) * dtdy
-          + (-w * dwz - (dpz + A * dAz + B * dBz) / r) * dtdz;
+    T su0, sv0, sw0;
+    auto velocity_sources = [&](auto &m) {
+        const auto ir = m.rec(r);
+        auto per_r = [&](T x) { return m.div(x, r, ir); };
+        su0 = (-u * dux - per_r(dpx + B * dBx + C * dCx)) * dtdx + (-v * duy + per_r(B * dAy)) * dtdy
+            + (-w * duz + per_r(C * dAz)) * dtdz;
+        sv0 = (-u * dvx + per_r(A * dBx)) * dtdx + (-v * dvy - per_r(dpy + A * dAy + C * dCy)) * dtdy
+            + (-w * dvz + per_r(C * dBz)) * dtdz;
+        sw0 = (-u * dwx + per_r(A * dCx)) * dtdx + (-v * dwy + per_r(B * dCy)) * dtdy
+            + (-w * dwz - per_r(dpz + A * dAz + B * dBz)) * dtdz;
+    };
+    if constexpr (sizeof(T) == 8) {
+        // nine quotients by the density from one reciprocal; again with the operators where an
+        // operand lies outside the range of round64.cuh
+        FastMath m;
+        velocity_sources(m);
+        if (m.bad()) {
+            IeeeMath e;
+            velocity_sources(e);
+        }
+    } else {
+        RecipMath m;
+        velocity_sources(m);
+    }
     T sp0 = (-u * dpx - dux * gamma * p) * dtdx + (-v * dpy - dvy * gamma * p) * dtdy
           + (-w * dpz - dwz * gamma * p) * dtdz;
     T sA0 = (u * dBy + B * duy - v * dAy - A * dvy) * dtdy + (u * dCz + C * duz - w * dAz - A * dwz) * dtdz;
@@ -719,10 +737,23 @@ constexpr int kTX = 32, kTY = kThreads / kTX;
 constexpr int kTR = kTX + 2;              // row of a staged plane (halo of one cell each side)
 constexpr int kTP = kTR * (kTY + 2);      // one field of a staged plane
 constexpr int kRingQ = 4, kRingE = 2;
-#ifndef DG_TRACE_KZ
-#define DG_TRACE_KZ 16
-#endif
-constexpr int kTZ = DG_TRACE_KZ;
+// A block marches through kz planes; its start costs about kTraceFill planes more (the fetch of three
+// planes with nothing to compute meanwhile).  kz is the march of at most 16 planes that needs the
+// least time by that count over the waves of resident blocks: 10 to 16 planes on large grids (10, 16
+// and 29 take the same time at 256^3), fewer where marches that long leave most of the chip idle
+// (FP64, both parts, always 16 planes -> this rule: 32 x 64 x 32 cells 0.104 -> 0.039 ms, 64^3 0.117 ->
+// 0.073, 101 x 75 x 53 0.127 -> 0.092; FP32, 32 x 64 x 32 cells: 0.054 -> 0.021).
+constexpr double kTraceFill = 2.5;
+inline int trace_march(int tiles, int planes, int slots) {
+    int best = 1;
+    double least = 1e300;
+    for (int kz = 1; kz <= 16 && kz <= planes; kz++) {
+        const long long blocks = (long long)tiles * ((planes + kz - 1) / kz);
+        const double cost = (double)((blocks + slots - 1) / slots) * (kz + kTraceFill);
+        if (cost <= least) { least = cost; best = kz; }
+    }
+    return best;
+}
 // staged fields of a cell plane; field v (0-7 primitives, 8-10 face-B components) sits at
 // slot position tq_pos(v): part 0 all 11, part 1 the 8 primitives, part 2 u, v, w and the face B
 template <int kPart> __host__ __device__ constexpr int tq_count() { return kPart == 0 ? NVAR + 3 : kPart == 1 ? NVAR : 6; }
@@ -731,24 +762,32 @@ template <int kPart> __host__ __device__ constexpr int tq_field(int f) {  // the
 }
 template <int kPart> __host__ __device__ constexpr int tq_pos(int v) { return kPart == 2 ? (v < NVAR ? v - IU : v - NVAR + 3) : v; }
 template <int kPart> __host__ __device__ constexpr bool t_edges() { return kPart != 1; }
+// part 1 also reads six face-field values of its own cell; each thread fetches the five new ones of
+// the next plane into slots of its own (C at k+1 is C at k of the next plane).  Loaded where they are
+// used, they were the part's largest stall; with the slots and the quotients of round64.cuh the FP64
+// trace takes 2.44 ms at 256^3 instead of 2.72.
+constexpr int kOwnF = 5;
 template <typename T, int kPart>
 constexpr int trace_tile_smem() {
-    return (kRingQ * tq_count<kPart>() + (t_edges<kPart>() ? kRingE * 3 : 0)) * kTP * (int)sizeof(T);
+    return (kRingQ * tq_count<kPart>() + (t_edges<kPart>() ? kRingE * 3 : 0)) * kTP * (int)sizeof(T) +
+           (kPart == 1 ? kOwnF * kThreads * (int)sizeof(T) : 0);
 }
 
 template <typename T, int kPart>
 struct TStencil {
     const T *p0, *p1, *p2;  // this cell in the staged cell planes k-1, k, k+1
     const T *e0, *e1;       // this cell in the edge planes k, k+1
-    const T *bg;            // part 1: this cell's left-face component 0 in global memory ...
-    long long sv, sy, sz;   // ... and the strides from it
+    T fb[6];                // part 1: A at i and i+1, B at j and j+1, C at k and k+1
     __device__ __forceinline__ const T *pl(int dk) const { return dk < 0 ? p0 : (dk > 0 ? p2 : p1); }
     __device__ __forceinline__ T q(int v, int di, int dj, int dk) const {
         if constexpr (kPart == 2) return T(0);  // part 2 evaluates no primitive
         else return pl(dk)[tq_pos<kPart>(v) * kTP + dj * kTR + di];
     }
     __device__ __forceinline__ T bf(int c, int di, int dj, int dk) const {
-        if constexpr (kPart == 1) return ld(bg + sv * c + sy * dj + sz * dk + di);
+        if constexpr (kPart == 1) {  // other offsets belong to the face slopes, which part 1 does not write
+            const int n = c == 0 ? di : c == 1 ? dj : dk;
+            return n == 0 || n == 1 ? fb[2 * c + n] : T(0);
+        }
         else return pl(dk)[tq_pos<kPart>(NVAR + c) * kTP + dj * kTR + di];
     }
     __device__ __forceinline__ T ex(int dj, int dk) const {
@@ -765,6 +804,14 @@ struct TStencil {
     }
 };
 
+template <typename T>
+__device__ __forceinline__ void cp_elem(T *dst, const T *src) {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(dst);
+    if constexpr (sizeof(T) == 4)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(a), "l"(src) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(a), "l"(src) : "memory");
+}
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
@@ -806,15 +853,8 @@ __device__ __forceinline__ void fetch_qplane(const Geo &G, const T *Q, const T *
         for (int f = 0; f < tq_count<kPart>(); f++) {
             const int v = tq_field<kPart>(f);
             const T *src = (v < NVAR ? Q + G.sv * v : Bf + G.sv * (IA + v - NVAR)) + c;
-            if (kok && P.in[n] && chk(src, sizeof(T))) {
-                const unsigned a = (unsigned)__cvta_generic_to_shared(d + f * kTP);
-                if constexpr (sizeof(T) == 4)
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(a), "l"(src) : "memory");
-                else
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(a), "l"(src) : "memory");
-            } else {
-                d[f * kTP] = T(0);
-            }
+            if (kok && P.in[n] && chk(src, sizeof(T))) cp_elem(d + f * kTP, src);
+            else d[f * kTP] = T(0);
         }
     }
 }
@@ -896,14 +936,14 @@ constexpr int trace_tile_minb() {
 }
 template <typename T, int kPart = 0>
 __global__ void __launch_bounds__(kThreads, (trace_tile_minb<T, kPart>()))
-k_trace3d_tile(Geo G, const T *__restrict__ Q, const T *__restrict__ Bf, T *__restrict__ core, const Scalars *S) {
+k_trace3d_tile(Geo G, int kz, const T *__restrict__ Q, const T *__restrict__ Bf, T *__restrict__ core, const Scalars *S) {
     extern __shared__ __align__(16) unsigned char tsm[];
     constexpr int kQS = tq_count<kPart>() * kTP;  // one cell-plane slot
     T *ringQ = (T *)tsm;
     T *ringE = ringQ + kRingQ * kQS;
     const int i0 = blockIdx.x * kTX, j0 = blockIdx.y * kTY;
-    const int kb = G.kc0 + blockIdx.z * kTZ;
-    const int ke = min(kb + kTZ, G.kc0 + G.CZ);  // core planes [kb, ke)
+    const int kb = G.kc0 + blockIdx.z * kz;
+    const int ke = min(kb + kz, G.kc0 + G.CZ);  // core planes [kb, ke)
     const int tx = threadIdx.x % kTX, ty = threadIdx.x / kTX;
     const int i = i0 + tx, j = j0 + ty;
     const bool mine = i < G.CX && j < G.CY;
@@ -911,6 +951,21 @@ k_trace3d_tile(Geo G, const T *__restrict__ Q, const T *__restrict__ Bf, T *__re
     auto qslot = [&](int k) { return ringQ + ((k - kb + 1) % kRingQ) * kQS; };
     auto eslot = [&](int k) { return ringE + ((k - kb) % kRingE) * (3 * kTP); };
     const double dtd = S->dt;
+    // part 1: this thread's own face-field slots; plane k's values, and C at k + 1
+    T *own_f = ringQ + kRingQ * kQS + threadIdx.x;
+    auto fetch_own = [&](int k) {
+        const T *a = Bf + G.sv * IA + G.idx(i, j, k);
+        const T *src[kOwnF] = {a, a + 1, a + G.sv, a + G.sv + G.sy, a + 2 * G.sv + G.sz};
+#pragma unroll
+        for (int n = 0; n < kOwnF; n++)
+            if (chk(src[n], sizeof(T))) cp_elem(own_f + n * kThreads, src[n]);
+    };
+    T c_left = T(0);
+    if constexpr (kPart == 1)
+        if (mine) {
+            c_left = ld(Bf + G.sv * IC + G.idx(i, j, kb));
+            fetch_own(kb);
+        }
     const FetchPos P = fetch_positions(G, i0, j0, kb - 1);
     fetch_qplane<T, kPart>(G, Q, Bf, qslot(kb - 1), P, kb - 1);
     fetch_qplane<T, kPart>(G, Q, Bf, qslot(kb), P, kb);
@@ -930,13 +985,21 @@ k_trace3d_tile(Geo G, const T *__restrict__ Q, const T *__restrict__ Bf, T *__re
             __syncthreads();
         }
         if (mine) {
-            TStencil<T, kPart> a{qslot(k - 1) + own, qslot(k) + own, qslot(k + 1) + own, nullptr, nullptr,
-                                 nullptr, G.sv, G.sy, G.sz};
+            TStencil<T, kPart> a{qslot(k - 1) + own, qslot(k) + own, qslot(k + 1) + own, nullptr, nullptr, {}};
             if constexpr (t_edges<kPart>()) {
                 a.e0 = eslot(k) + own;
                 a.e1 = eslot(k + 1) + own;
             }
-            if constexpr (kPart == 1) a.bg = Bf + G.sv * IA + G.idx(i, j, k);
+            if constexpr (kPart == 1) {
+#pragma unroll
+                for (int n = 0; n < 4; n++) a.fb[n] = own_f[n * kThreads];
+                a.fb[4] = c_left;
+                a.fb[5] = c_left = own_f[4 * kThreads];
+                if (k + 1 < ke) {
+                    fetch_own(k + 1);  // the slots are read: they take the next plane's values
+                    cp_commit();
+                }
+            }
             const long long t = (long long)i + (long long)G.CX * ((long long)j + (long long)G.CY * (k - G.kc0));
             trace3_cell<T, kPart>(a, G, i, dtd, core + core_base(t, kCore3));
         }
@@ -959,9 +1022,10 @@ cudaError_t launch_trace_tile(const Geo &G, const T *Q, const T *Bf, T *core, co
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
-    const dim3 grid((unsigned)((G.CX + kTX - 1) / kTX), (unsigned)((G.CY + kTY - 1) / kTY),
-                    (unsigned)((G.CZ + kTZ - 1) / kTZ));
-    k_trace3d_tile<T, kPart><<<grid, kThreads, smem, s>>>(G, Q, Bf, core, S);
+    const int tx = (G.CX + kTX - 1) / kTX, ty = (G.CY + kTY - 1) / kTY;
+    const int kz = trace_march(tx * ty, G.CZ, 148 * trace_tile_minb<T, kPart>());
+    const dim3 grid((unsigned)tx, (unsigned)ty, (unsigned)((G.CZ + kz - 1) / kz));
+    k_trace3d_tile<T, kPart><<<grid, kThreads, smem, s>>>(G, kz, Q, Bf, core, S);
     return cudaSuccess;
 }
 
