@@ -52,22 +52,21 @@ const char *kSlotNames[dg::KS_COUNT] = {"scalars", "cfl_dt", "primitive", "trace
 namespace {
 // the launch set of one arithmetic
 struct Launches {
-    int (*set_scalars)(const dg::Bufs &, double, double, int, int, cudaStream_t);
-    int (*advance_time)(const dg::Bufs &, cudaStream_t);
+    int (*set_scalars)(const dg::Geo &, const dg::Bufs &, double, double, int, int, cudaStream_t);
     int (*dt)(const dg::Geo &, const dg::Bufs &, int, cudaStream_t);
     int (*godunov)(const dg::Geo &, const dg::Bufs &, int, cudaStream_t);
     int (*fargo)(const dg::Geo &, const dg::Bufs &, int, cudaStream_t);
-    int (*boundary)(const dg::Geo &, const dg::Bufs &, int, cudaStream_t);
+    int (*boundary)(const dg::Geo &, const dg::Bufs &, int, cudaStream_t, int);
     int (*history)(const dg::Geo &, const dg::Bufs &, int, cudaStream_t, int);
     int (*history_columns)(const dg::Geo &, const dg::Bufs &, int, cudaStream_t);
     int (*history_share)(const dg::Geo &, const dg::Bufs &, int, cudaStream_t);
-    int (*dissipation)(const dg::Geo &, const dg::Bufs &, int, cudaStream_t);
+    int (*dissipation)(const dg::Geo &, const dg::Bufs &, int, cudaStream_t, int);
     int (*right_faces)(const dg::Geo &, const dg::Bufs &, int, double *, cudaStream_t);
     int (*to_f64)(const dg::Geo &, const dg::Bufs &, int, double *, cudaStream_t);
     int (*from_f64)(const dg::Geo &, const dg::Bufs &, int, const double *, int, cudaStream_t);
 };
 #define DG_LAUNCH_TABLE(ns)                                                                                  \
-    Launches{ns::launch_set_scalars, ns::launch_advance_time, ns::launch_dt, ns::launch_godunov, ns::launch_fargo, \
+    Launches{ns::launch_set_scalars, ns::launch_dt, ns::launch_godunov, ns::launch_fargo, \
              ns::launch_boundary, ns::launch_history, ns::launch_history_columns, ns::launch_history_share,   \
              ns::launch_dissipation, ns::launch_right_faces,                                                 \
              ns::launch_state_to_f64, ns::launch_f64_to_state}
@@ -400,11 +399,15 @@ int dg_init(const dg_params *p, dg_ctx **out) {
     {
         cudaError_t e = cudaMalloc((void **)&c->B.S, sizeof(dg::Scalars));
         if (e != cudaSuccess) return bail(fail(DG_ERR_NOMEM, "cudaMalloc of the device scalars failed"));
-        cudaMemsetAsync(c->B.S, 0, sizeof(dg::Scalars), c->stream);
     }
     if (cudaMallocHost((void **)&c->h_scal, sizeof(dg::Scalars)) != cudaSuccess ||
         cudaMallocHost((void **)&c->h_hist, 16 * sizeof(double)) != cudaSuccess)
         return bail(fail(DG_ERR_NOMEM, "cudaMallocHost failed"));
+    // the first CFL pass's minimum starts here; every pass leaves it so for the next
+    std::memset(c->h_scal, 0, sizeof(dg::Scalars));
+    c->h_scal->red = dg::cfl_start(G);
+    if (cudaMemcpyAsync(c->B.S, c->h_scal, sizeof(dg::Scalars), cudaMemcpyHostToDevice, c->stream) != cudaSuccess)
+        return bail(fail(DG_ERR_CUDA, "setting the device scalars failed"));
     if ((rc = bounded_sync(c->stream))) return bail(rc);
     for (auto &a : c->allocations) {  // no-ops unless the library is the bounds-checked build
         dg::f64::debug_register(a.first, a.second, 1);
@@ -727,7 +730,7 @@ int dg_godunov(dg_ctx *c, double dt, double time) {
     TimerScope ts_(c);
     if (!c) return fail(DG_ERR_ARG, "null context");
     if (!(dt > 0) || !std::isfinite(dt)) return fail(DG_ERR_DT, "dt must be positive and finite");
-    c->launches += c->L->set_scalars(c->B, dt, time, 1, 1, c->stream);
+    c->launches += c->L->set_scalars(c->G, c->B, dt, time, 1, 1, c->stream);
     c->B.q_fresh = (c->q_version == c->version);
     c->launches += c->L->godunov(c->G, c->B, c->cur, c->stream);
     c->cur ^= 1;
@@ -739,7 +742,7 @@ int dg_fargo_update(dg_ctx *c, double dt) {
     TimerScope ts_(c);
     if (!c) return fail(DG_ERR_ARG, "null context");
     if (!c->p.fargo) return fail(DG_ERR_ARG, "context was created with fargo = 0");
-    c->launches += c->L->set_scalars(c->B, dt, 0.0, 1, 0, c->stream);
+    c->launches += c->L->set_scalars(c->G, c->B, dt, 0.0, 1, 0, c->stream);
     c->launches += c->L->fargo(c->G, c->B, c->cur, c->stream);
     c->cur ^= 1;
     c->version++;
@@ -749,8 +752,8 @@ int dg_fargo_update(dg_ctx *c, double dt) {
 int dg_boundary(dg_ctx *c, double time, double dt) {
     TimerScope ts_(c);
     if (!c) return fail(DG_ERR_ARG, "null context");
-    c->launches += c->L->set_scalars(c->B, dt, time, 1, 1, c->stream);
-    c->launches += c->L->boundary(c->G, c->B, c->cur, c->stream);
+    c->launches += c->L->set_scalars(c->G, c->B, dt, time, 1, 1, c->stream);
+    c->launches += c->L->boundary(c->G, c->B, c->cur, c->stream, 0);
     c->version++;
     return check_launch();
 }
@@ -759,8 +762,8 @@ int dg_dissipation(dg_ctx *c, double time, double dt) {
     TimerScope ts_(c);
     if (!c) return fail(DG_ERR_ARG, "null context");
     if (!(c->G.nu > 0.0) && !(c->G.eta > 0.0)) return DG_OK;  // dumses.f90:104 calls it only then
-    c->launches += c->L->set_scalars(c->B, dt, time, 1, 1, c->stream);
-    c->launches += c->L->dissipation(c->G, c->B, c->cur, c->stream);
+    c->launches += c->L->set_scalars(c->G, c->B, dt, time, 1, 1, c->stream);
+    c->launches += c->L->dissipation(c->G, c->B, c->cur, c->stream, 0);
     c->version++;
     return check_launch();
 }
@@ -772,7 +775,7 @@ int dg_run(dg_ctx *c, int nsteps, double *time, double *dt) {
     if (c->G.nzslice > 1)
         return fail(DG_ERR_UNSUPPORTED, "a z slab needs its halos exchanged every step: drive it with dg_compute_dt, "
                                         "dg_godunov, dg_fargo_update, dg_boundary and dg_halo_pack/unpack");
-    c->launches += c->L->set_scalars(c->B, 0.0, *time, 0, 1, c->stream);
+    c->launches += c->L->set_scalars(c->G, c->B, 0.0, *time, 0, 1, c->stream);
     for (int n = 0; n < nsteps; n++) {
         c->launches += c->L->dt(c->G, c->B, c->cur, c->stream);
         c->B.q_fresh = 1;  // Q holds primitive(0) of this state from the CFL pass
@@ -782,10 +785,10 @@ int dg_run(dg_ctx *c, int nsteps, double *time, double *dt) {
             c->launches += c->L->fargo(c->G, c->B, c->cur, c->stream);
             c->cur ^= 1;
         }
-        c->launches += c->L->boundary(c->G, c->B, c->cur, c->stream);
-        if (c->G.nu > 0.0 || c->G.eta > 0.0) c->launches += c->L->dissipation(c->G, c->B, c->cur, c->stream);
+        const bool diss = c->G.nu > 0.0 || c->G.eta > 0.0;  // the last boundary call of the step advances time
+        c->launches += c->L->boundary(c->G, c->B, c->cur, c->stream, !diss);
+        if (diss) c->launches += c->L->dissipation(c->G, c->B, c->cur, c->stream, 1);
         c->version++;
-        c->launches += c->L->advance_time(c->B, c->stream);
     }
     int rc = check_launch();
     if (rc) return rc;

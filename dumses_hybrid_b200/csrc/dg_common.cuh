@@ -8,6 +8,7 @@
 // are bit-identical to a gfortran x86-64 build of the reference.
 #pragma once
 #include <cstdint>
+#include <cstring>
 #include <cuda_runtime.h>
 
 #include "dumses_gpu.h"
@@ -128,9 +129,24 @@ struct Scalars {
     double time;
     unsigned long long red;   // bits of the running CFL minimum (positive doubles order as integers)
     int err;                  // DG_ERR_* raised by a kernel (0 = none)
-    int sh_jp;                // shear offset of the x boundaries: whole cells ...
-    double sh_epsi;           // ... and remainder, for the time of the last k_shear_offset launch
+    unsigned done;            // blocks of the running CFL pass that have finished
+    // shear offset of the x boundaries: whole cells and remainder, [0] at time + dt / 2 (fluxes),
+    // [1] at time + dt (ghost cells); formed wherever dt or time is set
+    int sh_jp[2];
+    double sh_epsi[2];
 };
+
+// the bits of the CFL minimum's start, courant * dx / smallc (physics.f90:40)
+__host__ __device__ __forceinline__ unsigned long long cfl_start(const Geo &G) {
+    const double d0 = G.courant * G.dx / kSmallc;
+#ifdef __CUDA_ARCH__
+    return (unsigned long long)__double_as_longlong(d0);
+#else
+    unsigned long long b;
+    std::memcpy(&b, &d0, sizeof(b));
+    return b;
+#endif
+}
 
 // number of trace-core fields per cell
 constexpr int kCore3 = 47;

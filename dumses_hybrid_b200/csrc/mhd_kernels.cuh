@@ -50,18 +50,18 @@ extern thread_local KernelTimer *g_timer;  // set by the context that enqueues (
 
 // The launch set of one arithmetic; every function returns the number of kernels enqueued.
 #define DG_DECLARE_LAUNCHES                                                                          \
-    int launch_set_scalars(const Bufs &B, double dt, double time, int set_dt, int set_time, cudaStream_t st); \
-    int launch_advance_time(const Bufs &B, cudaStream_t st);                                         \
+    int launch_set_scalars(const Geo &G, const Bufs &B, double dt, double time, int set_dt, int set_time, cudaStream_t st); \
     int launch_dt(const Geo &G, const Bufs &B, int cur, cudaStream_t st);                            \
     int launch_godunov(const Geo &G, const Bufs &B, int cur, cudaStream_t st);   /* U[cur] -> U[cur^1] */ \
     int launch_fargo(const Geo &G, const Bufs &B, int cur, cudaStream_t st);     /* U[cur] -> U[cur^1] */ \
-    int launch_boundary(const Geo &G, const Bufs &B, int cur, cudaStream_t st);  /* in place on U[cur] */ \
+    /* in place on U[cur]; advance = 1 ends a step: time += dt on the device */                       \
+    int launch_boundary(const Geo &G, const Bufs &B, int cur, cudaStream_t st, int advance);         \
     int launch_history(const Geo &G, const Bufs &B, int cur, cudaStream_t st, int variant);          \
     /* z slabs: per-column sums of v_x, v_y into B.part (2 nx doubles); then this slab's share of */ \
     /* the history with the box's column means read from B.part, into B.hist */                      \
     int launch_history_columns(const Geo &G, const Bufs &B, int cur, cudaStream_t st);               \
     int launch_history_share(const Geo &G, const Bufs &B, int cur, cudaStream_t st);                 \
-    int launch_dissipation(const Geo &G, const Bufs &B, int cur, cudaStream_t st); /* in place, then boundary */ \
+    int launch_dissipation(const Geo &G, const Bufs &B, int cur, cudaStream_t st, int advance); /* in place, then boundary */ \
     int launch_right_faces(const Geo &G, const Bufs &B, int cur, double *out, cudaStream_t st);      \
     int launch_state_to_f64(const Geo &G, const Bufs &B, int cur, double *out, cudaStream_t st);     \
     int launch_f64_to_state(const Geo &G, const Bufs &B, int b, const double *in, int nv, cudaStream_t st); \

@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(kThreads, DG_UPDATE_MINB32) k_update3d_hl(Geo 
     const long long c = G.idx(i, j, k);
     const bool shear = G.shearing != 0;
     ShearRemap sr{0.0, 0};
-    if (shear) sr = ShearRemap{S->sh_epsi, S->sh_jp};  // time + dt/2, from k_shear_offset
+    if (shear) sr = ShearRemap{S->sh_epsi[0], S->sh_jp[0]};  // time + dt/2
     // the 8 pairs of the cell (c lies inside the ghosted grid for every face cell)
     float uh[8], ul[8];
 #pragma unroll
@@ -239,7 +239,7 @@ __device__ __forceinline__ void prim_hl(const Geo &G, const StoreHL &U, long lon
     }
 }
 
-__global__ void __launch_bounds__(kThreads) k_prim_hl(Geo G, StoreHL U, float *__restrict__ Q, const Scalars *S) {
+__global__ void __launch_bounds__(kThreads) k_prim_hl(Geo G, StoreHL U, float *__restrict__ Q) {
     const int ni = G.nx + 5, nj = (G.ndim > 1) ? G.ny + 5 : 1, nk = (G.ndim == 3) ? G.nz + 5 : 1;
     const long long n = (long long)ni * nj * nk;
     long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -252,12 +252,6 @@ __global__ void __launch_bounds__(kThreads) k_prim_hl(Geo G, StoreHL U, float *_
     const long long c = G.idx(i, j, k);
     float q[8];
     prim_hl(G, U, c, q);
-    if (G.omega0 > 0.0) {  // rotation half-kick, scheme.f90:78-85
-        const float om = (float)G.omega0, hdt = 0.5f * (float)S->dt;
-        const float dvx = 2.0f * om * q[IV], dvy = -(0.5f * om * q[IU]);
-        q[IU] = q[IU] + dvx * hdt;
-        q[IV] = q[IV] + dvy * hdt;
-    }
 #pragma unroll
     for (int v = 0; v < 8; v++) Q[G.sv * v + c] = q[v];
 }
@@ -265,7 +259,7 @@ __global__ void __launch_bounds__(kThreads) k_prim_hl(Geo G, StoreHL U, float *_
 // compute_dt fused with the primitive variables of the next godunov: one pass over the
 // ghosted grid writes Q without the rotation half-kick (prim_hl) and reduces the CFL time
 // step over the active cells (FP32 signal speeds from prim_hl, the minimum of the per-cell
-// time steps taken on their bit patterns); k_kick adds the half-kick once dt is known
+// time steps taken on their bit patterns); the trace adds the half-kick once dt is known
 __global__ void __launch_bounds__(kThreads) k_prim_dt_hl(Geo G, StoreHL U, float *__restrict__ Q, Scalars *S) {
     const int ni = G.nx + 5, nj = (G.ndim > 1) ? G.ny + 5 : 1, nk = (G.ndim == 3) ? G.nz + 5 : 1;
     const long long n = (long long)ni * nj * nk;
@@ -274,8 +268,7 @@ __global__ void __launch_bounds__(kThreads) k_prim_dt_hl(Geo G, StoreHL U, float
     const float vsh = ((G.omega0 > 0.0) && !G.fargo) ? (float)(1.5 * G.omega0 * (G.xmax - G.xmin) * 0.5) : 0.0f;
     float best = __int_as_float(0x7f800000);  // +inf
     int bad = 0;
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t < n) {
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
         int i, j, k;
         split3((unsigned)t, G.dPX, G.dPY, i, j, k);
         i -= 2;
@@ -309,22 +302,8 @@ __global__ void __launch_bounds__(kThreads) k_prim_dt_hl(Geo G, StoreHL U, float
     if (threadIdx.x == 0) {
         unsigned long long m = sb[0];
         for (int w = 1; w < kThreads / 32; w++) m = sb[w] < m ? sb[w] : m;
-        // one block per 128 cells: skip the atomic when the running minimum is already smaller
-        if (m < *(volatile unsigned long long *)&S->red) atomicMin(&S->red, m);
+        finish_dt(G, S, m);
     }
-}
-
-// rotation half-kick (scheme.f90:78-85) on the primitive velocities of the ghosted grid:
-// one thread per element of the velocity planes, the never-read outer ghost layer included,
-// so no cell index is decomposed
-__global__ void __launch_bounds__(kThreads) k_kick(Geo G, float *__restrict__ Q, const Scalars *S) {
-    const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (c >= G.sv) return;
-    const float om = (float)G.omega0, hdt = 0.5f * (float)S->dt;
-    const float u = Q[G.sv * IU + c], v = Q[G.sv * IV + c];
-    const float dvx = 2.0f * om * v, dvy = -(0.5f * om * u);
-    Q[G.sv * IU + c] = u + dvx * hdt;
-    Q[G.sv * IV + c] = v + dvy * hdt;
 }
 
 // ---------------------------------------------------------------------------
@@ -848,35 +827,17 @@ StoreHL st(const Bufs &B, int b) {
         if (g_timer) g_timer->end(slot, st);             \
     } while (0)
 
-int launch_set_scalars(const Bufs &B, double dt, double time, int set_dt, int set_time, cudaStream_t s) {
-    TIMED(KS_SCALARS, s, (k_set_scalars<<<1, 1, 0, s>>>(B.S, dt, time, set_dt, set_time)));
-    return 1;
-}
-
-int launch_advance_time(const Bufs &B, cudaStream_t s) {
-    TIMED(KS_SCALARS, s, (k_advance_time<<<1, 1, 0, s>>>(B.S)));
+int launch_set_scalars(const Geo &G, const Bufs &B, double dt, double time, int set_dt, int set_time, cudaStream_t s) {
+    TIMED(KS_SCALARS, s, (k_set_scalars<<<1, 1, 0, s>>>(G, B.S, dt, time, set_dt, set_time)));
     return 1;
 }
 
 int launch_dt(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
-    TIMED(KS_DT, s, (k_dt_reset<<<1, 1, 0, s>>>(G, B.S)));
     // the primitive variables of godunov come out of the same pass (Q without the half-kick)
     const long long ng = (long long)(G.nx + 5) * ((G.ndim > 1) ? G.ny + 5 : 1) * ((G.ndim == 3) ? G.nz + 5 : 1);
-    TIMED(KS_DT, s, (k_prim_dt_hl<<<nblocks(ng, kThreads), kThreads, 0, s>>>(G, st(B, cur), (float *)B.Q, B.S)));
-    TIMED(KS_DT, s, (k_dt_final<<<1, 1, 0, s>>>(G, B.S)));
-    return 3;
+    TIMED(KS_DT, s, (k_prim_dt_hl<<<mn(nblocks(ng, kThreads), kDtBlocks), kThreads, 0, s>>>(G, st(B, cur), (float *)B.Q, B.S)));
+    return 1;
 }
-
-// 3D trace as two kernels: cell fields, then face fields
-#ifndef DG_TRACE_SPLIT32
-#define DG_TRACE_SPLIT32 0
-#endif
-constexpr bool kTraceSplit32 = DG_TRACE_SPLIT32 != 0;
-// 3D trace with its stencil staged in shared memory (k_trace3d_tile)
-#ifndef DG_TRACE_TILE32
-#define DG_TRACE_TILE32 1
-#endif
-constexpr bool kTraceTile32 = DG_TRACE_TILE32 != 0;
 
 // 3D Riemann work as two kernels (faces, then edges) instead of one
 #ifndef DG_RIEMANN_SPLIT32
@@ -887,40 +848,26 @@ constexpr bool kRiemannSplit32 = DG_RIEMANN_SPLIT32 != 0;
 int launch_godunov(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
     const StoreHL U = st(B, cur), Un = st(B, cur ^ 1);
     float *Q = (float *)B.Q, *core = (float *)B.core;
-    float *E0 = (float *)B.E[0], *E1 = (float *)B.E[1], *E2 = (float *)B.E[2];
+    float *E2 = (float *)B.E[2];
     float *fx = (float *)B.flx[0], *fy = (float *)B.flx[1], *fz = (float *)B.flx[2];
     float *ex = (float *)B.emf[0], *ey = (float *)B.emf[1], *ez = (float *)B.emf[2];
     const int ni = G.nx + 5, nj = (G.ndim > 1) ? G.ny + 5 : 1, nk = (G.ndim == 3) ? G.nz + 5 : 1;
-    int n = (G.shearing ? 1 : 0) + 4;
-    if (!B.q_fresh) {
-        TIMED(KS_PRIM, s, (k_prim_hl<<<nblocks((long long)ni * nj * nk, kThreads), kThreads, 0, s>>>(G, U, Q, B.S)));
-        n++;
-    } else if (G.omega0 > 0.0) {  // Q of this state from launch_dt: add the rotation half-kick
-        TIMED(KS_PRIM, s, (k_kick<<<nblocks(G.sv, kThreads), kThreads, 0, s>>>(G, Q, B.S)));
+    int n = 3;
+    if (!B.q_fresh) {  // else Q of this state from launch_dt
+        TIMED(KS_PRIM, s, (k_prim_hl<<<nblocks((long long)ni * nj * nk, kThreads), kThreads, 0, s>>>(G, U, Q)));
         n++;
     }
-    if (G.shearing) TIMED(KS_SCALARS, s, (k_shear_offset<<<1, 1, 0, s>>>(G, B.S, 0.5)));
+    if (G.omega0 > 0.0 && G.ndim < 3) {
+        TIMED(KS_PRIM, s, (k_kick<float><<<nblocks(G.sv, kThreads), kThreads, 0, s>>>(G, Q, B.S)));
+        n++;
+    }
     int faces = 1;
     if (G.ndim == 3) {
-        // the tiled trace computes its edge fields itself
-        if (kTraceTile32) n--;
-        else TIMED(KS_EFIELD, s, (k_efield3d<float><<<nblocks(G.esz, kThreads), kThreads, 0, s>>>(G, Q, U.hi, E0, E1, E2)));
-        if (kTraceTile32 && kTraceSplit32) {
-            TIMED(KS_TRACE, s, (launch_trace_tile<float, 1>(G, Q, U.hi, core, B.S, s)));
-            TIMED(KS_TRACE, s, (launch_trace_tile<float, 2>(G, Q, U.hi, core, B.S, s)));
-            n++;
-        } else if (kTraceTile32) {
-            TIMED(KS_TRACE, s, (launch_trace_tile<float>(G, Q, U.hi, core, B.S, s)));
-        } else if (kTraceSplit32) {
-            TIMED(KS_TRACE, s, (k_trace3d<float, 1><<<nblocks(G.csz, kThreads), kThreads, 0, s>>>(G, Q, U.hi, E0, E1, E2, core, B.S)));
-            TIMED(KS_TRACE, s, (k_trace3d<float, 2><<<nblocks(G.csz, kThreads), kThreads, 0, s>>>(G, Q, U.hi, E0, E1, E2, core, B.S)));
-            n++;
-        } else {
-            TIMED(KS_TRACE, s, (k_trace3d<float><<<nblocks(G.csz, kThreads), kThreads, 0, s>>>(G, Q, U.hi, E0, E1, E2, core, B.S)));
-        }
+        TIMED(KS_TRACE, s, (launch_trace_tile<float, 0>(G, Q, U.hi, core, B.S, s)));
     } else {
         TIMED(KS_EFIELD, s, (k_efield2d<float><<<nblocks(G.esz, kThreads), kThreads, 0, s>>>(G, Q, U.hi, E2)));
         TIMED(KS_TRACE, s, (k_trace2d<float><<<nblocks(G.csz, kThreads), kThreads, 0, s>>>(G, Q, U.hi, E2, core, B.S)));
+        n++;
     }
     float *fl[3] = {fx, fy, fz};
     if (B.net) {
@@ -975,7 +922,8 @@ int launch_trace_only(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
     float *Q = (float *)B.Q, *core = (float *)B.core;
     float *E0 = (float *)B.E[0], *E1 = (float *)B.E[1], *E2 = (float *)B.E[2];
     const int ni = G.nx + 5, nj = (G.ndim > 1) ? G.ny + 5 : 1, nk = (G.ndim == 3) ? G.nz + 5 : 1;
-    TIMED(KS_PRIM, s, (k_prim_hl<<<nblocks((long long)ni * nj * nk, kThreads), kThreads, 0, s>>>(G, U, Q, B.S)));
+    TIMED(KS_PRIM, s, (k_prim_hl<<<nblocks((long long)ni * nj * nk, kThreads), kThreads, 0, s>>>(G, U, Q)));
+    if (G.omega0 > 0.0) TIMED(KS_PRIM, s, (k_kick<float><<<nblocks(G.sv, kThreads), kThreads, 0, s>>>(G, Q, B.S)));
     if (G.ndim == 3) {
         TIMED(KS_EFIELD, s, (k_efield3d<float><<<nblocks(G.esz, kThreads), kThreads, 0, s>>>(G, Q, U.hi, E0, E1, E2)));
         TIMED(KS_TRACE, s, (k_trace3d<float><<<nblocks(G.csz, kThreads), kThreads, 0, s>>>(G, Q, U.hi, E0, E1, E2, core, B.S)));
@@ -983,7 +931,7 @@ int launch_trace_only(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
         TIMED(KS_EFIELD, s, (k_efield2d<float><<<nblocks(G.esz, kThreads), kThreads, 0, s>>>(G, Q, U.hi, E2)));
         TIMED(KS_TRACE, s, (k_trace2d<float><<<nblocks(G.csz, kThreads), kThreads, 0, s>>>(G, Q, U.hi, E2, core, B.S)));
     }
-    return 3;
+    return 3 + (G.omega0 > 0.0);
 }
 
 const void *nn_faces_kernel() { return (const void *)k_nn_faces; }
@@ -1008,14 +956,9 @@ int launch_fargo(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
     return 2;
 }
 
-int launch_boundary(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
-    int n = 1;
-    if (G.shearing) {
-        TIMED(KS_SCALARS, s, (k_shear_offset<<<1, 1, 0, s>>>(G, B.S, 1.0)));
-        n++;
-    }
-    TIMED(KS_BOUNDARY, s, (k_boundary<StoreHL><<<nblocks(ghost_cells(G), kThreads), kThreads, 0, s>>>(G, st(B, cur), B.nv, B.S)));
-    return n;
+int launch_boundary(const Geo &G, const Bufs &B, int cur, cudaStream_t s, int advance) {
+    TIMED(KS_BOUNDARY, s, (k_boundary<StoreHL><<<nblocks(ghost_cells(G), kThreads), kThreads, 0, s>>>(G, st(B, cur), B.nv, B.S, advance)));
+    return 1;
 }
 
 int launch_right_faces(const Geo &G, const Bufs &B, int cur, double *out, cudaStream_t s) {
@@ -1036,7 +979,7 @@ int launch_f64_to_state(const Geo &G, const Bufs &B, int b, const double *in, in
 
 // dissipation (physics.f90:272-291): resistive EMFs + CT, viscous fluxes + update, in
 // place on U[cur], then boundary; the step's EMF and flux arrays are free at this point
-int launch_dissipation(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
+int launch_dissipation(const Geo &G, const Bufs &B, int cur, cudaStream_t s, int advance) {
     const StoreHL U = st(B, cur);
     float *e0 = (float *)B.emf[0], *e1 = (float *)B.emf[1], *e2 = (float *)B.emf[2];
     float *f0 = (float *)B.flx[0], *f1 = (float *)B.flx[1], *f2 = G.ndim == 3 ? (float *)B.flx[2] : f0;
@@ -1056,7 +999,7 @@ int launch_dissipation(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
         TIMED(KS_DISSIPATION, s, (k_visc_update<StoreHL><<<nb, kThreads, 0, s>>>(G, U, f0, f1, f2)));
         n += 3;
     }
-    return n + launch_boundary(G, B, cur, s);
+    return n + launch_boundary(G, B, cur, s, advance);
 }
 
 int launch_history(const Geo &G, const Bufs &B, int cur, cudaStream_t s, int variant) {

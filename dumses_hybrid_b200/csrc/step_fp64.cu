@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(kThreads) k_update3d(
     if (!chk(Un + c, 8) || !chk(Un + sv * IC + c, 8)) return;  // the planes this thread writes
     const bool shear = G.shearing != 0;
     ShearRemap sr{0.0, 0};
-    if (shear) sr = ShearRemap{S->sh_epsi, S->sh_jp};  // time + dt/2, from k_shear_offset
+    if (shear) sr = ShearRemap{S->sh_epsi[0], S->sh_jp[0]};  // time + dt/2
 
     if (i <= nx && j <= ny && k <= nz) {
         // hydro update, scheme.f90:1783-1907
@@ -310,84 +310,39 @@ StoreD st(const Bufs &B, int b) { return StoreD{(double *)B.U[b]}; }
         if (g_timer) g_timer->end(slot, st);             \
     } while (0)
 
-int launch_set_scalars(const Bufs &B, double dt, double time, int set_dt, int set_time, cudaStream_t s) {
-    TIMED(KS_SCALARS, s, (k_set_scalars<<<1, 1, 0, s>>>(B.S, dt, time, set_dt, set_time)));
-    return 1;
-}
-
-int launch_advance_time(const Bufs &B, cudaStream_t s) {
-    TIMED(KS_SCALARS, s, (k_advance_time<<<1, 1, 0, s>>>(B.S)));
+int launch_set_scalars(const Geo &G, const Bufs &B, double dt, double time, int set_dt, int set_time, cudaStream_t s) {
+    TIMED(KS_SCALARS, s, (k_set_scalars<<<1, 1, 0, s>>>(G, B.S, dt, time, set_dt, set_time)));
     return 1;
 }
 
 // compute_dt; the pass also leaves primitive(0) in Q for the godunov that follows (B.q_fresh)
 int launch_dt(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
-    TIMED(KS_DT, s, (k_dt_reset<<<1, 1, 0, s>>>(G, B.S)));
     const int ni = G.nx + 5, nj = (G.ndim > 1) ? G.ny + 5 : 1, nk = (G.ndim == 3) ? G.nz + 5 : 1;
-    TIMED(KS_DT, s, (k_prim_dt<StoreD><<<nblocks((long long)ni * nj * nk, kThreads), kThreads, 0, s>>>(G, st(B, cur), (double *)B.Q, B.S)));
-    TIMED(KS_DT, s, (k_dt_final<<<1, 1, 0, s>>>(G, B.S)));
-    return 3;
+    TIMED(KS_DT, s, (k_prim_dt<StoreD><<<mn(nblocks((long long)ni * nj * nk, kThreads), kDtBlocks), kThreads, 0, s>>>(G, st(B, cur), (double *)B.Q, B.S)));
+    return 1;
 }
-
-// the rotation half-kick of primitive(dt) on Q = primitive(0), as prim_cell applies it
-// (scheme.f90:78-85): one thread per element of the velocity planes
-__global__ void __launch_bounds__(kThreads) k_kick64(Geo G, double *__restrict__ Q, const Scalars *S) {
-    const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (c >= G.sv) return;
-    const double half = 0.5, two = 2.0, dt = S->dt;
-    const double u = Q[G.sv * IU + c], v = Q[G.sv * IV + c];
-    const double dvx = two * G.omega0 * v;
-    const double dvy = -(half * G.omega0 * u);
-    Q[G.sv * IU + c] = u + dvx * dt * half;
-    Q[G.sv * IV + c] = v + dvy * dt * half;
-}
-
-// 3D trace as two kernels: cell fields (5 blocks per SM, 96 registers), then face fields
-// (6 blocks per SM); 3.03 against 3.68 ms at 256^3 for the single kernel, which spills at 128
-#ifndef DG_TRACE_SPLIT64
-#define DG_TRACE_SPLIT64 1
-#endif
-constexpr bool kTraceSplit64 = DG_TRACE_SPLIT64 != 0;
-// 3D trace with its stencil staged in shared memory (k_trace3d_tile)
-#ifndef DG_TRACE_TILE64
-#define DG_TRACE_TILE64 1
-#endif
-constexpr bool kTraceTile64 = DG_TRACE_TILE64 != 0;
 
 int launch_godunov(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
     const StoreD U = st(B, cur);
     double *Un = (double *)B.U[cur ^ 1];
     double *Q = (double *)B.Q, *core = (double *)B.core;
-    double *E0 = (double *)B.E[0], *E1 = (double *)B.E[1], *E2 = (double *)B.E[2];
+    double *E2 = (double *)B.E[2];
     double *fx = (double *)B.flx[0], *fy = (double *)B.flx[1], *fz = (double *)B.flx[2];
     double *ex = (double *)B.emf[0], *ey = (double *)B.emf[1], *ez = (double *)B.emf[2];
     const int ni = G.nx + 5, nj = (G.ndim > 1) ? G.ny + 5 : 1, nk = (G.ndim == 3) ? G.nz + 5 : 1;
-    int n = 4 + (G.shearing ? 1 : 0);
-    if (!B.q_fresh) {
-        TIMED(KS_PRIM, s, (k_prim<double, StoreD><<<nblocks((long long)ni * nj * nk, kThreads), kThreads, 0, s>>>(G, U, Q, B.S)));
-        n++;
-    } else if (G.omega0 > 0.0) {  // Q = primitive(0) of this state from launch_dt: add the half-kick
-        TIMED(KS_PRIM, s, (k_kick64<<<nblocks(G.sv, kThreads), kThreads, 0, s>>>(G, Q, B.S)));
+    int n = 3;
+    if (!B.q_fresh) {  // else Q = primitive(0) of this state from launch_dt
+        TIMED(KS_PRIM, s, (k_prim<double, StoreD><<<nblocks((long long)ni * nj * nk, kThreads), kThreads, 0, s>>>(G, U, Q)));
         n++;
     }
-    if (G.shearing) TIMED(KS_SCALARS, s, (k_shear_offset<<<1, 1, 0, s>>>(G, B.S, 0.5)));
+    if (G.omega0 > 0.0 && G.ndim < 3) {
+        TIMED(KS_PRIM, s, (k_kick<double><<<nblocks(G.sv, kThreads), kThreads, 0, s>>>(G, Q, B.S)));
+        n++;
+    }
     if (G.ndim == 3) {
-        // the tiled trace computes its edge fields itself
-        if (kTraceTile64) n--;
-        else TIMED(KS_EFIELD, s, (k_efield3d<double><<<nblocks(G.esz, kThreads), kThreads, 0, s>>>(G, Q, U.p, E0, E1, E2)));
-        if (kTraceTile64 && kTraceSplit64) {
-            TIMED(KS_TRACE, s, (launch_trace_tile<double, 1>(G, Q, U.p, core, B.S, s)));
-            TIMED(KS_TRACE, s, (launch_trace_tile<double, 2>(G, Q, U.p, core, B.S, s)));
-            n++;
-        } else if (kTraceTile64) {
-            TIMED(KS_TRACE, s, (launch_trace_tile<double>(G, Q, U.p, core, B.S, s)));
-        } else if (kTraceSplit64) {
-            TIMED(KS_TRACE, s, (k_trace3d<double, 1><<<nblocks(G.csz, kThreads), kThreads, 0, s>>>(G, Q, U.p, E0, E1, E2, core, B.S)));
-            TIMED(KS_TRACE, s, (k_trace3d<double, 2><<<nblocks(G.csz, kThreads), kThreads, 0, s>>>(G, Q, U.p, E0, E1, E2, core, B.S)));
-            n++;
-        } else {
-            TIMED(KS_TRACE, s, (k_trace3d<double><<<nblocks(G.csz, kThreads), kThreads, 0, s>>>(G, Q, U.p, E0, E1, E2, core, B.S)));
-        }
+        TIMED(KS_TRACE, s, (launch_trace_tile<double, 1>(G, Q, U.p, core, B.S, s)));
+        TIMED(KS_TRACE, s, (launch_trace_tile<double, 2>(G, Q, U.p, core, B.S, s)));
+        n++;
         // HLLD/HLLD (the reference's default and every benchmark) runs its own kernel, the other
         // solvers one kernel for the faces and one for the edges
         const unsigned nb = nblocks(G.fsz, kThreads);
@@ -407,12 +362,12 @@ int launch_godunov(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
         if (hlld) TIMED(KS_RIEMANN, s, (k_riemann1d<double, true><<<nblocks(G.FX, kThreads), kThreads, 0, s>>>(G, core, fx, B.S)));
         else TIMED(KS_RIEMANN, s, (k_riemann1d<double, false><<<nblocks(G.FX, kThreads), kThreads, 0, s>>>(G, core, fx, B.S)));
         TIMED(KS_UPDATE, s, (k_update1d<<<nblocks(G.nx, kThreads), kThreads, 0, s>>>(G, U.p, Un, fx, B.S)));
-        n--;
     } else {
         TIMED(KS_EFIELD, s, (k_efield2d<double><<<nblocks(G.esz, kThreads), kThreads, 0, s>>>(G, Q, U.p, E2)));
         TIMED(KS_TRACE, s, (k_trace2d<double><<<nblocks(G.csz, kThreads), kThreads, 0, s>>>(G, Q, U.p, E2, core, B.S)));
         TIMED(KS_RIEMANN, s, (k_riemann2d<double><<<nblocks(G.fsz, kThreads), kThreads, 0, s>>>(G, core, fx, fy, ez, B.S, 1)));
         TIMED(KS_UPDATE, s, (k_update2d<<<nblocks(G.fsz, kThreads), kThreads, 0, s>>>(G, U.p, Un, fx, fy, ez, B.S)));
+        n++;
     }
     return n;
 }
@@ -423,14 +378,9 @@ int launch_fargo(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
     return 2;
 }
 
-int launch_boundary(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
-    int n = 1;
-    if (G.shearing) {
-        TIMED(KS_SCALARS, s, (k_shear_offset<<<1, 1, 0, s>>>(G, B.S, 1.0)));
-        n++;
-    }
-    TIMED(KS_BOUNDARY, s, (k_boundary<StoreD><<<nblocks(ghost_cells(G), kThreads), kThreads, 0, s>>>(G, st(B, cur), B.nv, B.S)));
-    return n;
+int launch_boundary(const Geo &G, const Bufs &B, int cur, cudaStream_t s, int advance) {
+    TIMED(KS_BOUNDARY, s, (k_boundary<StoreD><<<nblocks(ghost_cells(G), kThreads), kThreads, 0, s>>>(G, st(B, cur), B.nv, B.S, advance)));
+    return 1;
 }
 
 int launch_right_faces(const Geo &G, const Bufs &B, int cur, double *out, cudaStream_t s) {
@@ -465,7 +415,7 @@ int launch_history_ptrs(const Geo &G, const double *U, double *scratch, double *
 
 // dissipation (physics.f90:272-291): resistive EMFs + CT, viscous fluxes + update, in
 // place on U[cur], then boundary; the step's EMF and flux arrays are free at this point
-int launch_dissipation(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
+int launch_dissipation(const Geo &G, const Bufs &B, int cur, cudaStream_t s, int advance) {
     const StoreD U = st(B, cur);
     double *e0 = (double *)B.emf[0], *e1 = (double *)B.emf[1], *e2 = (double *)B.emf[2];
     double *f0 = (double *)B.flx[0], *f1 = (double *)B.flx[1], *f2 = G.ndim == 3 ? (double *)B.flx[2] : f0;
@@ -485,7 +435,7 @@ int launch_dissipation(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
         TIMED(KS_DISSIPATION, s, (k_visc_update<StoreD><<<nb, kThreads, 0, s>>>(G, U, f0, f1, f2)));
         n += 3;
     }
-    return n + launch_boundary(G, B, cur, s);
+    return n + launch_boundary(G, B, cur, s, advance);
 }
 
 __global__ void k_history_1d(Geo G, const double *__restrict__ U, double *__restrict__ out) {

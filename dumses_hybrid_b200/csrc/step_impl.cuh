@@ -12,7 +12,7 @@
 //   k_prim_dt     compute_dt  (physics.f90:18-132)      primitive(0) into Q + CFL min-reduction
 //   k_prim        primitive   (scheme.f90:20-91)        Q on the ghosted grid
 //   k_efield      edge E of trace3d/trace2d (scheme.f90:1194-1239, 856-872), once per edge
-//   k_trace       slope + trace3d/trace2d (scheme.f90:253-656, 807-1711)
+//   k_trace       slope + trace3d/trace2d (scheme.f90:253-656, 807-1711), with primitive(dt)'s half-kick
 //                 -> per-cell "trace core": predicted cell state, half slopes,
 //                    predicted face B and its transverse half slopes; every
 //                    face and corner state of the reference is one add (and a
@@ -213,26 +213,54 @@ struct StoreHL {
 // ---------------------------------------------------------------------------
 // small scalar kernels
 // ---------------------------------------------------------------------------
-__global__ void k_set_scalars(Scalars *S, double dt, double time, int set_dt, int set_time) {
+struct ShearRemap {
+    double epsi;
+    int jp;
+};
+// shear offset of the x boundaries at time itime (shearingbox.f90:34-37)
+__device__ __forceinline__ ShearRemap shear_offset(const Geo &G, double itime) {
+    double deltay = 1.5 * G.omega0 * (G.xmax - G.xmin) * itime;
+    deltay = fmod(deltay, (G.ymax - G.ymin));
+    ShearRemap s;
+    s.epsi = fmod(deltay, G.dy);
+    s.jp = (int)(deltay / G.dy);
+    return s;
+}
+// the offsets of the step whose dt and time S holds
+__device__ __forceinline__ void set_shear(const Geo &G, Scalars *S) {
+    if (!G.shearing) return;
+    for (int n = 0; n < 2; n++) {
+        const ShearRemap r = shear_offset(G, S->time + (n ? 1.0 : 0.5) * S->dt);
+        S->sh_jp[n] = r.jp;
+        S->sh_epsi[n] = r.epsi;
+    }
+}
+
+__global__ void k_set_scalars(Geo G, Scalars *S, double dt, double time, int set_dt, int set_time) {
     if (set_dt) S->dt = dt;
     if (set_time) S->time = time;
+    set_shear(G, S);
 }
 
-__global__ void k_advance_time(Scalars *S) { S->time = S->time + S->dt; }
-
-__global__ void k_dt_reset(Geo G, Scalars *S) {
-    // dt = courant*dx/smallc before the minimum (physics.f90:40)
-    double d0 = G.courant * G.dx / kSmallc;
-    S->red = (unsigned long long)__double_as_longlong(d0);
-}
-
-__global__ void k_dt_final(Geo G, Scalars *S) {
-    double m = __longlong_as_double((long long)S->red);
-    double dt = G.courant * m;
-    if (!(dt > 0.0) || !isfinite(dt)) S->err = DG_ERR_DT;
+// The end of a CFL pass: every block brings its minimum m (bit pattern); the last one to finish forms dt and the shear offsets and leaves S ready for the next pass.
+// (Three launches of one thread each did this before: 64^3 Orszag-Tang CFL pass 29 -> 19 us.)  The
+// pass runs on a grid of kDtBlocks blocks that stride over the cells: with a block per 128 cells the
+// counter's atomics alone took 0.07 ms at 256^3.
+constexpr unsigned kDtBlocks = 148 * 16;
+__device__ __forceinline__ void finish_dt(const Geo &G, Scalars *S, unsigned long long m) {
+    if (m < *(volatile unsigned long long *)&S->red) atomicMin(&S->red, m);
+    __threadfence();
+    if (atomicAdd(&S->done, 1u) != gridDim.x - 1) return;
+    __threadfence();
+    const double dt = G.courant * __longlong_as_double((long long)*(volatile unsigned long long *)&S->red);
+    int err = *(volatile int *)&S->err;
+    if (!(dt > 0.0) || !isfinite(dt)) S->err = err = DG_ERR_DT;
     // after a failed CFL pass (a non-finite state, or no valid step) the steps that dg_run has
     // already enqueued behind it run with dt = 0 and change nothing; the host reports the error
-    S->dt = S->err ? 0.0 : dt;
+    S->dt = err ? 0.0 : dt;
+    S->red = cfl_start(G);
+    S->done = 0;
+    set_shear(G, S);
 }
 
 // primitive variables of one cell in FP64 (scheme.f90:44-86); the right faces are the
@@ -283,16 +311,15 @@ __device__ __forceinline__ double comp_speed(double gamma, double rho, double p,
 // compute_dt (physics.f90:42-121) fused with the primitive variables of the next godunov
 // (FP64 path): one pass over the ghosted grid writes Q = primitive(0) (prim_cell with dt = 0,
 // no rotation half-kick) and reduces the CFL time step over the active cells; the
-// half-kick of primitive(dt) (scheme.f90:78-85) is added once dt is known (k_kick64), to the
-// same unkicked values in the same order, so Q ends as primitive(dt) bit for bit
+// half-kick of primitive(dt) (scheme.f90:78-85) is added once dt is known, by the trace (kick), to the
+// same unkicked values in the same order as primitive(dt) does
 template <class Store>
 __global__ void __launch_bounds__(kThreads) k_prim_dt(Geo G, Store U, double *__restrict__ Q, Scalars *S) {
     const int ni = G.nx + 5, nj = (G.ndim > 1) ? G.ny + 5 : 1, nk = (G.ndim == 3) ? G.nz + 5 : 1;
     const long long n = (long long)ni * nj * nk;
     double best = __longlong_as_double(0x7ff0000000000000LL);  // +inf
     int bad = 0;
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t < n) {
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
         int i, j, k;
         split3((unsigned)t, G.dPX, G.dPY, i, j, k);
         i -= 2;
@@ -337,16 +364,16 @@ __global__ void __launch_bounds__(kThreads) k_prim_dt(Geo G, Store U, double *__
     if (threadIdx.x == 0) {
         unsigned long long m = sb[0];
         for (int w = 1; w < kThreads / 32; w++) m = sb[w] < m ? sb[w] : m;
-        // one block per 128 cells: skip the atomic when the running minimum is already smaller
-        if (m < *(volatile unsigned long long *)&S->red) atomicMin(&S->red, m);
+        finish_dt(G, S, m);
     }
 }
 
 // ---------------------------------------------------------------------------
-// primitive variables on the ghosted grid (cells with a right neighbour)
+// primitive variables on the ghosted grid (cells with a right neighbour), without the rotation
+// half-kick
 // ---------------------------------------------------------------------------
 template <typename T, class Store>
-__global__ void __launch_bounds__(kThreads) k_prim(Geo G, Store U, T *__restrict__ Q, const Scalars *S) {
+__global__ void __launch_bounds__(kThreads) k_prim(Geo G, Store U, T *__restrict__ Q) {
     const int ni = G.nx + 5, nj = (G.ndim > 1) ? G.ny + 5 : 1, nk = (G.ndim == 3) ? G.nz + 5 : 1;
     const long long n = (long long)ni * nj * nk;
     long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -358,9 +385,35 @@ __global__ void __launch_bounds__(kThreads) k_prim(Geo G, Store U, T *__restrict
     k = (G.ndim == 3) ? k - 2 : 1;
     const long long c = G.idx(i, j, k);
     double q[8];
-    prim_cell(G, U, c, S->dt, q);
+    prim_cell(G, U, c, 0.0, q);
 #pragma unroll
     for (int v = 0; v < 8; v++) Q[G.sv * v + c] = (T)q[v];
+}
+
+// rotation half-kick of the predicted velocities (scheme.f90:78-85)
+__device__ __forceinline__ void kick(const Geo &G, double dt, double &u, double &v) {
+    const double half = 0.5, two = 2.0;
+    const double dvx = two * G.omega0 * v;
+    const double dvy = -(half * G.omega0 * u);
+    u = u + dvx * dt * half;
+    v = v + dvy * dt * half;
+}
+__device__ __forceinline__ void kick(const Geo &G, double dtd, float &u, float &v) {
+    const float om = (float)G.omega0, hdt = 0.5f * (float)dtd;
+    const float dvx = 2.0f * om * v, dvy = -(0.5f * om * u);
+    u = u + dvx * hdt;
+    v = v + dvy * hdt;
+}
+// the same on the velocity planes of Q, one thread per element (2D and 1D; the 3D trace adds it to
+// the planes it stages)
+template <typename T>
+__global__ void __launch_bounds__(kThreads) k_kick(Geo G, T *__restrict__ Q, const Scalars *S) {
+    const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (c >= G.sv) return;
+    T u = Q[G.sv * IU + c], v = Q[G.sv * IV + c];
+    kick(G, S->dt, u, v);
+    Q[G.sv * IU + c] = u;
+    Q[G.sv * IV + c] = v;
 }
 
 // the slope limiter of slope() for slope_type 1 and 2 (scheme.f90:450-458)
@@ -518,27 +571,6 @@ __device__ __forceinline__ T face_slope(const QV<T> &a, int c, int dir, int i, i
 #ifndef DG_RIEMANN_MINB32
 #define DG_RIEMANN_MINB32 8
 #endif
-// kPart selects the core fields a launch writes: 0 all 47; 1 the predicted cell state and the
-// cell slopes (fields 0-28); 2 the predicted face fields and their transverse slopes (29-46).
-// The values a part does not write are not computed (their expressions are dead code), and
-// every written value is the same expression of the same inputs in all forms.
-#ifndef DG_TRACEC_MINB64
-#define DG_TRACEC_MINB64 5
-#endif
-#ifndef DG_TRACEF_MINB64
-#define DG_TRACEF_MINB64 6
-#endif
-#ifndef DG_TRACEC_MINB32
-#define DG_TRACEC_MINB32 6
-#endif
-#ifndef DG_TRACEF_MINB32
-#define DG_TRACEF_MINB32 8
-#endif
-template <typename T, int kPart>
-constexpr int trace_minb() {
-    return sizeof(T) == 8 ? (kPart == 0 ? DG_TRACE_MINB64 : kPart == 1 ? DG_TRACEC_MINB64 : DG_TRACEF_MINB64)
-                          : (kPart == 0 ? DG_TRACE_MINB32 : kPart == 1 ? DG_TRACEC_MINB32 : DG_TRACEF_MINB32);
-}
 // The 3D trace of one cell (slope + trace3d, scheme.f90:253-656, 1149-1711) written once over a
 // stencil accessor that reads, relative to the cell (i, j, k):
 //   a.q(v, di, dj, dk)   primitive variable v of cell (i+di, j+dj, k+dk)
@@ -706,8 +738,8 @@ __device__ __forceinline__ void trace3_cell(const Sten &a, const Geo &G, int i, 
     }
 }
 
-template <typename T, int kPart = 0>
-__global__ void __launch_bounds__(kThreads, (trace_minb<T, kPart>()))
+template <typename T>
+__global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 ? DG_TRACE_MINB64 : DG_TRACE_MINB32))
 k_trace3d(Geo G, const T *__restrict__ Q, const T *__restrict__ Bf, const T *__restrict__ Exa,
           const T *__restrict__ Eya, const T *__restrict__ Eza, T *__restrict__ core, const Scalars *S) {
     long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -716,7 +748,7 @@ k_trace3d(Geo G, const T *__restrict__ Q, const T *__restrict__ Bf, const T *__r
     split3((unsigned)t, G.dCX, G.dCY, i, j, k);
     k += G.kc0;
     const GStencil<T> a{QV<T>{Q, Bf, G}, Exa, Eya, Eza, i, j, k};
-    trace3_cell<T, kPart>(a, G, i, S->dt, core + core_base(t, kCore3));
+    trace3_cell<T, 0>(a, G, i, S->dt, core + core_base(t, kCore3));
 }
 
 // ---------------------------------------------------------------------------
@@ -859,6 +891,21 @@ __device__ __forceinline__ void fetch_qplane(const Geo &G, const T *Q, const T *
     }
 }
 
+// the rotation half-kick on the positions of a staged plane that this thread fetched
+template <typename T, int kPart>
+__device__ __forceinline__ void kick_plane(const Geo &G, T *s, const FetchPos &P, double dtd) {
+    constexpr int pU = tq_pos<kPart>(IU) * kTP, pV = tq_pos<kPart>(IV) * kTP;
+#pragma unroll
+    for (int n = 0; n < 2; n++) {
+        if (P.q[n] < 0) continue;
+        T *c = s + P.q[n];
+        T u = c[pU], v = c[pV];
+        kick(G, dtd, u, v);
+        c[pU] = u;
+        c[pV] = v;
+    }
+}
+
 // the trace's edge fields of plane k (Ex_at, Ey_at, Ez_at on the staged cell planes lo = k-1
 // and hi = k) for the edges i0..i0+kTX, j0..j0+kTY, into slot s at the cells' positions
 template <typename T, int kPart>
@@ -909,39 +956,18 @@ __device__ __forceinline__ void edge_plane(const Geo &G, const T *lo, const T *h
     }
 }
 
-// resident blocks per SM the tiled trace is compiled for, by arithmetic and part (bounded by
-// its shared memory: FP64 82/52/49 KB, FP32 41/26/24 KB per block for parts 0/1/2)
-#ifndef DG_TRACET_MINB64
-#define DG_TRACET_MINB64 2
-#endif
-#ifndef DG_TRACET1_MINB64
-#define DG_TRACET1_MINB64 4
-#endif
-#ifndef DG_TRACET2_MINB64
-#define DG_TRACET2_MINB64 4
-#endif
-#ifndef DG_TRACET_MINB32
-#define DG_TRACET_MINB32 5
-#endif
-#ifndef DG_TRACET1_MINB32
-#define DG_TRACET1_MINB32 6
-#endif
-#ifndef DG_TRACET2_MINB32
-#define DG_TRACET2_MINB32 8
-#endif
+// resident blocks per SM the tiled trace is compiled for (bounded by its shared memory: 56 KB per
+// block in FP64, 41 KB in FP32)
+template <typename T>
+constexpr int trace_tile_minb() { return sizeof(T) == 8 ? 4 : 5; }
 template <typename T, int kPart>
-constexpr int trace_tile_minb() {
-    return sizeof(T) == 8 ? (kPart == 0 ? DG_TRACET_MINB64 : kPart == 1 ? DG_TRACET1_MINB64 : DG_TRACET2_MINB64)
-                          : (kPart == 0 ? DG_TRACET_MINB32 : kPart == 1 ? DG_TRACET1_MINB32 : DG_TRACET2_MINB32);
-}
-template <typename T, int kPart = 0>
-__global__ void __launch_bounds__(kThreads, (trace_tile_minb<T, kPart>()))
-k_trace3d_tile(Geo G, int kz, const T *__restrict__ Q, const T *__restrict__ Bf, T *__restrict__ core, const Scalars *S) {
+__device__ __forceinline__ void trace_tile(const Geo &G, int tile_x, int kz, const T *Q, const T *Bf, T *core, double dtd) {
     extern __shared__ __align__(16) unsigned char tsm[];
     constexpr int kQS = tq_count<kPart>() * kTP;  // one cell-plane slot
     T *ringQ = (T *)tsm;
     T *ringE = ringQ + kRingQ * kQS;
-    const int i0 = blockIdx.x * kTX, j0 = blockIdx.y * kTY;
+    const int i0 = tile_x * kTX, j0 = blockIdx.y * kTY;
+    const bool rotating = G.omega0 > 0.0;
     const int kb = G.kc0 + blockIdx.z * kz;
     const int ke = min(kb + kz, G.kc0 + G.CZ);  // core planes [kb, ke)
     const int tx = threadIdx.x % kTX, ty = threadIdx.x / kTX;
@@ -950,7 +976,6 @@ k_trace3d_tile(Geo G, int kz, const T *__restrict__ Q, const T *__restrict__ Bf,
     const int own = (ty + 1) * kTR + (tx + 1);  // this cell in a staged plane
     auto qslot = [&](int k) { return ringQ + ((k - kb + 1) % kRingQ) * kQS; };
     auto eslot = [&](int k) { return ringE + ((k - kb) % kRingE) * (3 * kTP); };
-    const double dtd = S->dt;
     // part 1: this thread's own face-field slots; plane k's values, and C at k + 1
     T *own_f = ringQ + kRingQ * kQS + threadIdx.x;
     auto fetch_own = [&](int k) {
@@ -973,6 +998,8 @@ k_trace3d_tile(Geo G, int kz, const T *__restrict__ Q, const T *__restrict__ Bf,
     fetch_qplane<T, kPart>(G, Q, Bf, qslot(kb + 1), P, kb + 1);
     cp_commit();
     cp_wait_all();
+    if (rotating)
+        for (int k = kb - 1; k <= kb + 1; k++) kick_plane<T, kPart>(G, qslot(k), P, dtd);
     __syncthreads();
     if constexpr (t_edges<kPart>()) edge_plane<T, kPart>(G, qslot(kb - 1), qslot(kb), eslot(kb), i0);
     for (int k = kb; k < ke; k++) {
@@ -1004,15 +1031,26 @@ k_trace3d_tile(Geo G, int kz, const T *__restrict__ Q, const T *__restrict__ Bf,
             trace3_cell<T, kPart>(a, G, i, dtd, core + core_base(t, kCore3));
         }
         cp_wait_all();
+        if (rotating && k + 2 <= ke) kick_plane<T, kPart>(G, qslot(k + 2), P, dtd);
         __syncthreads();  // cell plane k+2 is in; every thread is done with planes k-1 (cells, edges)
     }
 }
 
-// launch k_trace3d_tile over the core index space (its dynamic shared memory is above the
-// default 48 KB limit in FP64: the attribute is set once per device)
-template <typename T, int kPart = 0>
+// The trace over the core index space: FP32 as part 0, FP64 as a launch of part 1 and one of part 2
+// (side by side in one grid the parts took 2.9 instead of 2.5 ms at 256^3: the larger part's
+// registers and shared memory for both).
+template <typename T, int kPart>
+__global__ void __launch_bounds__(kThreads, trace_tile_minb<T>())
+k_trace3d_tile(const __grid_constant__ Geo G, int kz, const T *__restrict__ Q, const T *__restrict__ Bf,
+               T *__restrict__ core, const Scalars *S) {
+    trace_tile<T, kPart>(G, blockIdx.x, kz, Q, Bf, core, S->dt);
+}
+
+// launch k_trace3d_tile (its dynamic shared memory is above the default 48 KB limit in FP64: the
+// attribute is set once per device)
+template <typename T, int kPart>
 cudaError_t launch_trace_tile(const Geo &G, const T *Q, const T *Bf, T *core, const Scalars *S, cudaStream_t s) {
-    const int smem = trace_tile_smem<T, kPart>();
+    constexpr int smem = trace_tile_smem<T, kPart>();
     static bool attr_set[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -1023,7 +1061,7 @@ cudaError_t launch_trace_tile(const Geo &G, const T *Q, const T *Bf, T *core, co
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
     const int tx = (G.CX + kTX - 1) / kTX, ty = (G.CY + kTY - 1) / kTY;
-    const int kz = trace_march(tx * ty, G.CZ, 148 * trace_tile_minb<T, kPart>());
+    const int kz = trace_march(tx * ty, G.CZ, 148 * trace_tile_minb<T>());
     const dim3 grid((unsigned)tx, (unsigned)ty, (unsigned)((G.CZ + kz - 1) / kz));
     k_trace3d_tile<T, kPart><<<grid, kThreads, smem, s>>>(G, kz, Q, Bf, core, S);
     return cudaSuccess;
@@ -1661,20 +1699,6 @@ __global__ void __launch_bounds__(kThreads) k_riemann2d(Geo G, const T *__restri
 // ---------------------------------------------------------------------------
 // update + constrained transport
 // ---------------------------------------------------------------------------
-struct ShearRemap {
-    double epsi;
-    int jp;
-};
-// shear offset of the x boundaries at time itime (shearingbox.f90:34-37)
-__device__ __forceinline__ ShearRemap shear_offset(const Geo &G, double itime) {
-    double deltay = 1.5 * G.omega0 * (G.xmax - G.xmin) * itime;
-    deltay = fmod(deltay, (G.ymax - G.ymin));
-    ShearRemap s;
-    s.epsi = fmod(deltay, G.dy);
-    s.jp = (int)(deltay / G.dy);
-    return s;
-}
-
 // Any y index into [1, n].  Equal to the reference's single "+/- ny" wrap whenever
 // that wrap lands inside the active range; the reference reads a ghost row or
 // unallocated memory otherwise (a shift of a full box or more), which this guard
@@ -1683,13 +1707,6 @@ __device__ __forceinline__ int wrap1(int j, int n) {
     if (j >= 1 && j <= n) return j;
     int m = (j - 1) % n;
     return (m < 0 ? m + n : m) + 1;
-}
-
-// shear offset at time + frac*dt, computed once per step phase instead of per thread
-__global__ void k_shear_offset(Geo G, Scalars *S, double frac) {
-    const ShearRemap r = shear_offset(G, S->time + frac * S->dt);
-    S->sh_jp = r.jp;
-    S->sh_epsi = r.epsi;
 }
 
 // shearing_flux / shearing_emf average of a face quantity on the inner (side 0)
@@ -1742,9 +1759,10 @@ __host__ __device__ __forceinline__ long long ghost_cells(const Geo &G) {
 
 constexpr int kMaxVars = 10;  // stored state variables: 8, plus the frozen right-face B (z in 2D, y and z in 1D)
 template <class Store>
-__global__ void __launch_bounds__(kThreads) k_boundary(Geo G, Store U, int nv, const Scalars *S) {
+__global__ void __launch_bounds__(kThreads) k_boundary(Geo G, Store U, int nv, Scalars *S, int advance) {
     long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= ghost_cells(G)) return;
+    if (advance && t == 0) S->time = S->time + S->dt;  // the last kernel of a step; no thread here reads time
     // the ghost counts of any grid that fits a GPU are far below 2^32: 32-bit index arithmetic
     const unsigned NX = G.NX, NY = G.NY;
     const unsigned nA = (G.ndim == 3) ? 6u * NX * NY : 0u;
@@ -1790,8 +1808,8 @@ __global__ void __launch_bounds__(kThreads) k_boundary(Geo G, Store U, int nv, c
         return;
     }
     // shear-periodic x ghost (only with ndim = 3; shearingbox.f90:62-147): the remapped rows,
-    // eps and lambda are the same for every variable; offset for time+dt from k_shear_offset
-    const ShearRemap sr{S->sh_epsi, S->sh_jp};
+    // eps and lambda are the same for every variable; offset for time + dt
+    const ShearRemap sr{S->sh_epsi[1], S->sh_jp[1]};
     const int nx = G.nx, ny = G.ny;
     const double one = 1.0, half = 0.5;
     const bool lower = i < 1;
