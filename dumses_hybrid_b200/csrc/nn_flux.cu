@@ -34,6 +34,12 @@ __host__ __device__ constexpr int real_n(int l) { return l == kNHid ? kOut : kHi
 // transposed input (kInPad rows) or the transposed, zero-padded activations (kHidT rows)
 __host__ __device__ constexpr int dw_cols(int l) { return l == 0 ? kInPad : kHidT; }
 
+__host__ __device__ constexpr int param_count() {
+    int n = 0;
+    for (int l = 0; l < kNL; l++) n += real_k(l) * real_n(l) + real_n(l);
+    return n;
+}
+
 enum { M_FWD_HID = 0, M_FWD_OUT = 1, M_BWD_HID = 2, M_DW = 3 };
 
 constexpr int kGemmSmem = 65536 + 1024;  // A tile, B tile, barriers, bias sums (caps residency at 3 CTAs/SM)
@@ -276,10 +282,289 @@ __global__ void __launch_bounds__(128) k_loss(const float *__restrict__ Y, const
     }
 }
 
+// ---------------------------------------------------------------------------
+// One training pass (gather, forward, loss, backward, weight gradients) in one kernel.
+//
+// The pass was a chain of 10 kernels that handed BF16 operands, their transposed copies and the
+// activation derivatives to each other through HBM and spent their time in the epilogues' 2-byte and
+// strided stores and per-column shuffle sums: 156 us for a batch of 65536 (17-64-64-8), where the
+// products themselves are a few microseconds of tensor time (batch of 65536: an Adam step 206 us then,
+// 48 us now, 40 of them in this kernel).  Here a persistent block takes
+// 128-row tiles through the whole pass: the activations stay in shared memory as the operands of the
+// next product, the pre-activations stay in tensor memory for the backward pass, and the weight
+// gradients accumulate in tensor memory over the block's tiles.  Only the sampled rows are read and
+// one gradient per block is written.  Bound by the latency of its chain of products and epilogues:
+// four warpgroups share a tile, each with 16 of its columns, and the next tile's rows are in flight.
+//
+// Shared-memory operands are blocked K-major as in nn_umma.cuh.  The transposed operands (reduction
+// over the tile's 128 rows) hold kHid rows; as the A operand of an M = 128 product their rows kHid..127
+// are whatever follows in shared memory, and so are the tensor-memory lanes that no one reads.
+constexpr int kTrainBlocks = 148;
+constexpr int kTrainThreads = 512, kParts = kTrainThreads / kTileRows;
+constexpr int kTrainX = kInPad * kTileRows * 2, kTrainH = kHid * kTileRows * 2, kTrainD = kOutPad * kTileRows * 2;
+constexpr int train_weights() {  // bytes of the forward and backward weight operands
+    int b = 0;
+    for (int l = 0; l < kNL; l++) b += layer_k(l) * layer_n(l) * 2 * (l > 0 ? 2 : 1);
+    return b;
+}
+constexpr int kTrainSmem = 2 * kTrainX + (2 + kNHid) * kTrainH + 2 * kTrainD + train_weights() + 2048 + 1024;
+constexpr int kTrainCols = (kNHid + 1) * kHid + kOutPad + kOutPad + (kNHid - 1) * kHid + kInPad;  // tensor-memory columns
+// the shapes it is built for (default 17-64-64-8: 114 KB, 320 columns); others train by the kernel chain
+constexpr bool kTrainFused = kHid <= 64 && kTrainSmem <= 227 * 1024 && kTrainCols <= 512;
+
+struct TrainArgs {
+    const float *xs, *ts;
+    long long ns, rows, first;
+    int random;
+    unsigned long long seed;
+    const Scaling *sc;
+    const bf16 *Wt[kNL], *Wn[kNL];
+    const float *b[kNL];
+    float *part;   // [block][parameters] gradient sums
+    float *lpart;  // [block] loss sums
+    int *err;
+};
+
+// column sums over a warp: lane L returns the sum over all lanes of v[L >> 1] (each exchange
+// halves the columns a lane still carries)
+__device__ __forceinline__ float warp_column_sum16(float v[16], int lane) {
+#pragma unroll
+    for (int w = 8, o = 16; w > 0; w >>= 1, o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int q = 0; q < w; q++) {
+            const float keep = up ? v[q + w] : v[q], send = up ? v[q] : v[q + w];
+            v[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+// D (+)= A B^T over ksteps K = 16 steps; A's row count fixes its chunk stride
+__device__ __forceinline__ void mma_run(uint32_t d, const void *a, int arows, const void *b, int n, int ksteps, int acc) {
+    const unsigned al = arows * 16, bl = n * 16;
+    for (int s = 0; s < ksteps; s++)
+        mma_bf16(d, sdesc((const char *)a + (size_t)s * 2 * al, al, 128), sdesc((const char *)b + (size_t)s * 2 * bl, bl, 128),
+                 idesc_bf16(kTileRows, n), s > 0 || acc);
+}
+
+__global__ void __launch_bounds__(kTrainThreads, 1) k_train(const __grid_constant__ TrainArgs g) {
+    extern __shared__ __align__(1024) unsigned char sm[];
+    unsigned char *at = sm;
+    auto take = [&](int bytes) { unsigned char *p = at; at += bytes; return (bf16 *)p; };
+    bf16 *Xn = take(kTrainX), *Xt = take(kTrainX);
+    bf16 *Hn = take(kTrainH), *Dt = take(kTrainH), *Ht[kNHid];  // Hn also holds the backward pass's deltas
+    for (int l = 0; l < kNHid; l++) Ht[l] = take(kTrainH);
+    bf16 *On = take(kTrainD), *Ot = take(kTrainD), *Wt[kNL], *Wn[kNL];
+    for (int l = 0; l < kNL; l++) {
+        Wt[l] = take(layer_k(l) * layer_n(l) * 2);
+        Wn[l] = l > 0 ? take(layer_k(l) * layer_n(l) * 2) : nullptr;
+    }
+    float *red = (float *)take(2048);  // [16 warps][16 columns], rows past the operands for M = 128 reads
+    uint64_t *bar = (uint64_t *)take(1024);
+    uint32_t *tslot = (uint32_t *)(bar + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rl = tid & (kTileRows - 1), part = tid / kTileRows;  // row of the tile, and 16 columns of a layer
+    if (tid == 0) {
+        mbar_init(bar, 1);
+        mbar_fence_init();
+    }
+    if (warp == 0) tmem_alloc(tslot, 512);
+    for (int l = 0; l < kNL; l++) {
+        const int n16 = layer_k(l) * layer_n(l) / 8;
+        for (int q = tid; q < n16; q += kTrainThreads) {
+            ((uint4 *)Wt[l])[q] = ((const uint4 *)g.Wt[l])[q];
+            if (l > 0) ((uint4 *)Wn[l])[q] = ((const uint4 *)g.Wn[l])[q];
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tm = *tslot;
+    // tensor-memory columns: pre-activations, outputs, backward accumulator, weight gradients
+    const uint32_t zcol = tm, ocol = tm + kNHid * kHid, acol = ocol + kOutPad, gout = acol + kHid, ghid = gout + kOutPad;
+    auto gcol = [&](int l) { return l == kNHid ? gout : l == 0 ? ghid + (kNHid - 1) * kHid : ghid + (l - 1) * kHid; };
+    const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
+
+    unsigned phase = 0;
+    bool bad = false;
+    // make this tile's operands visible, have thread 0 issue the products, and wait for them
+    auto products = [&](auto issue) {
+        fence_async_smem();
+        tc_fence_before();
+        __syncthreads();
+        if (tid == 0) {
+            tc_fence_after();
+            issue();
+            mma_commit(bar);
+        }
+        if (!bad) bad = !mbar_wait(bar, phase);
+        phase ^= 1;
+        tc_fence_after();
+    };
+    const long long tiles = g.rows / kTileRows;
+    // this thread's 8 of the 32 padded input columns; the last part has only padding and takes the targets
+    const int x0 = part * 8;
+    float mu[8], isd[8], px[8], pt[kOut];
+    const bool targets = part == kParts - 1;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        mu[q] = x0 + q < kIn ? g.sc->xmu[x0 + q] : 0.0f;
+        isd[q] = x0 + q < kIn ? g.sc->xisd[x0 + q] : 0.0f;
+    }
+    auto fetch = [&](long long tile) {
+        const long long b = tile * kTileRows + rl;
+        const long long idx = g.random ? (long long)(mix64(g.seed ^ (unsigned long long)b * 0xD1B54A32D192ED03ull) % (unsigned long long)g.ns)
+                                       : g.first + b;
+        const bool in = idx < g.ns;
+#pragma unroll
+        for (int q = 0; q < 8; q++) px[q] = in && x0 + q < kIn ? g.xs[idx * kIn + x0 + q] : 0.0f;
+#pragma unroll
+        for (int q = 0; q < kOut; q++) pt[q] = in && targets ? g.ts[idx * kOut + q] : 0.0f;
+    };
+    fetch(blockIdx.x);
+    float bsum[kNHid], osum = 0.0f;  // this lane's running column sums: hidden biases; output biases and the loss
+#pragma unroll
+    for (int l = 0; l < kNHid; l++) bsum[l] = 0.0f;
+    // 16 values of this row (columns 16 part ..) as operands of the next product and, transposed, of a gradient
+    auto put = [&](const float v[16], bf16 *normal, bf16 *transposed) {
+        if (normal) {
+            store_bf16x8(normal + ((part * 2) * kTileRows + rl) * 8, v);
+            store_bf16x8(normal + ((part * 2 + 1) * kTileRows + rl) * 8, v + 8);
+        }
+        bf16 *t = transposed + ((rl >> 3) * kHid + part * 16) * 8 + (rl & 7);
+#pragma unroll
+        for (int q = 0; q < 16; q++) t[q * 8] = __float2bfloat16_rn(v[q]);
+    };
+    const bool hidden = part * 16 < kHid;  // this part has columns of a hidden layer
+    bool begun = false;
+    for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        {   // standardised inputs; zero columns past kIn
+            float x[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) x[q] = (px[q] - mu[q]) * isd[q];
+            store_bf16x8(Xn + (part * kTileRows + rl) * 8, x);
+            bf16 *t = Xt + ((rl >> 3) * kInPad + x0) * 8 + (rl & 7);
+#pragma unroll
+            for (int q = 0; q < 8; q++) t[q * 8] = __float2bfloat16_rn(x[q]);
+        }
+        float tgt[kOut];
+#pragma unroll
+        for (int q = 0; q < kOut; q++) tgt[q] = targets ? pt[q] / g.sc->ysd[q] : 0.0f;
+        if (tile + gridDim.x < tiles) fetch(tile + gridDim.x);
+        // forward
+#pragma unroll
+        for (int l = 0; l < kNHid; l++) {
+            products([&] { mma_run(zcol + l * kHid, l == 0 ? Xn : Hn, kTileRows, Wt[l], kHid, layer_k(l) / 16, 0); });
+            if (hidden) {
+                float v[16];
+                tmem_ld16(zcol + l * kHid + part * 16 + lanes, v);
+#pragma unroll
+                for (int q = 0; q < 16; q++) v[q] = smelu(v[q] + __ldg(g.b[l] + part * 16 + q));
+                put(v, Hn, Ht[l]);
+            }
+        }
+        products([&] { mma_run(ocol, Hn, kTileRows, Wt[kNHid], kOutPad, kHid / 16, 0); });
+        if (targets) {  // mean-squared-error gradient of the outputs, sums of the loss and the output biases
+            float v[16];
+            tmem_ld16(ocol + lanes, v);
+            const float sc = 2.0f / (float)(g.rows * kOut);
+            float l = 0.0f;
+#pragma unroll
+            for (int q = 0; q < kOut; q++) {
+                const float e = v[q] + __ldg(g.b[kNHid] + q) - tgt[q];
+                v[q] = sc * e;
+                l += e * e;
+            }
+#pragma unroll
+            for (int q = kOut; q < 16; q++) v[q] = 0.0f;
+            store_bf16x8(On + rl * 8, v);
+            store_bf16x8(On + (kTileRows + rl) * 8, v + 8);
+            bf16 *t = Ot + ((rl >> 3) * kOutPad) * 8 + (rl & 7);
+#pragma unroll
+            for (int q = 0; q < kOutPad; q++) t[q * 8] = __float2bfloat16_rn(v[q]);
+            v[kOut] = l;
+            osum += warp_column_sum16(v, lane);
+        }
+        // backward: deltas of layer l from those of layer l + 1, and the gradient of layer l + 1's weights
+#pragma unroll
+        for (int l = kNHid - 1; l >= 0; l--) {
+            products([&] {
+                if (l == kNHid - 1) {
+                    mma_run(acol, On, kTileRows, Wn[l + 1], kHid, kOutPad / 16, 0);
+                    mma_run(gcol(l + 1), Ht[l], kHid, Ot, kOutPad, kTileRows / 16, begun);
+                } else {
+                    mma_run(acol, Hn, kTileRows, Wn[l + 1], kHid, kHid / 16, 0);
+                    mma_run(gcol(l + 1), Dt, kHid, Ht[l], kHid, kTileRows / 16, begun);
+                }
+            });
+            if (hidden) {
+                float v[16], z[16];
+                tmem_ld16(acol + part * 16 + lanes, v);
+                tmem_ld16(zcol + l * kHid + part * 16 + lanes, z);
+#pragma unroll
+                for (int q = 0; q < 16; q++) v[q] *= smelu_d(z[q] + __ldg(g.b[l] + part * 16 + q));
+                put(v, l > 0 ? Hn : nullptr, Dt);
+                bsum[l] += warp_column_sum16(v, lane);
+            }
+        }
+        products([&] { mma_run(gcol(0), Dt, kHid, Xt, kInPad, kTileRows / 16, begun); });
+        begun = true;
+    }
+    // this block's gradient in parameter order: the weight gradients are [n][k] for the hidden layers
+    // (lane n, column k) and [k][n] for the output layer
+    float *out = g.part + blockIdx.x * (long long)param_count();
+    const int n = rl;
+#pragma unroll
+    for (int l = 0; l < kNL; l++) {
+        const int cols = l == kNHid ? kOutPad : l == 0 ? kInPad : kHid;
+        if (part * 16 < cols) {
+            float v[16];
+            tmem_ld16(gcol(l) + part * 16 + lanes, v);
+            if (n < kHid) {
+#pragma unroll
+                for (int q = 0; q < 16; q++) {
+                    const int k = part * 16 + q;
+                    if (l == kNHid) {
+                        if (k < kOut) out[n * kOut + k] = v[q];
+                    } else if (k < real_k(l)) {
+                        out[k * kHid + n] = v[q];
+                    }
+                }
+            }
+        }
+        out += real_k(l) * real_n(l) + real_n(l);
+    }
+    // biases: column sums of the four warps that hold a column
+    out = g.part + blockIdx.x * (long long)param_count();
+#pragma unroll
+    for (int l = 0; l < kNL; l++) {
+        out += real_k(l) * real_n(l);
+        __syncthreads();
+        if (!(lane & 1)) red[warp * 16 + (lane >> 1)] = l == kNHid ? osum : bsum[l < kNHid ? l : 0];
+        __syncthreads();
+        if (tid < (l == kNHid ? kOut + 1 : kHid)) {
+            const int w0 = l == kNHid ? 4 * (kParts - 1) : (tid >> 4) * 4, c = l == kNHid ? tid : tid & 15;
+            const float v = red[w0 * 16 + c] + red[(w0 + 1) * 16 + c] + red[(w0 + 2) * 16 + c] + red[(w0 + 3) * 16 + c];
+            if (l == kNHid && tid == kOut) g.lpart[blockIdx.x] = v;
+            else out[tid] = v;
+        }
+        out += real_n(l);
+    }
+    if (bad) atomicOr(g.err, NN_ERR_WAIT);
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after();
+        tmem_dealloc(tm, 512);
+    }
+}
+
 struct AdamArgs {
     float *W[kNL], *b[kNL], *mW[kNL], *vW[kNL], *mb[kNL], *vb[kNL];
     const float *dw[kNL];  // weight-gradient partials
     const float *db[kNL];  // bias-gradient partials
+    const float *part;     // or (not null) `splits` gradients in parameter order
     bf16 *Wt[kNL], *Wn[kNL], *Bt[kNHid];
     int splits, tiles;
     float lr, beta1, beta2, eps, c1, c2;  // c1 = 1 - beta1^t, c2 = 1 - beta2^t
@@ -289,13 +574,18 @@ struct AdamArgs {
 
 __host__ __device__ constexpr long long layer_params(int l) { return (long long)real_k(l) * real_n(l) + real_n(l); }
 
-// one thread per real parameter: reduce its gradient partials, Adam step on the FP32
-// master, BF16 copies in both operand layouts
-__global__ void k_adam(AdamArgs a) {
-    long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+// kAdamGroup threads per real parameter add its gradient partials (their loads coalesce over the 32
+// parameters of a block); the first of them does the Adam step on the FP32 master and writes the BF16
+// copies in both operand layouts.  One thread per parameter took 41 us for 128 splits: a serial chain
+// of loads on 23 blocks.
+constexpr int kAdamGroup = 8, kAdamParams = 32;
+__global__ void __launch_bounds__(kAdamGroup * kAdamParams) k_adam(AdamArgs a) {
+    const int col = threadIdx.x % kAdamParams, grp = threadIdx.x / kAdamParams;
+    long long t = blockIdx.x * (long long)kAdamParams + col;
     int l = 0;
     while (l < kNL && t >= layer_params(l)) { t -= layer_params(l); l++; }
-    if (l >= kNL) return;
+    const bool have = l < kNL;
+    if (!have) l = kNL - 1;
     long long off = 0;
     for (int q = 0; q < l; q++) off += layer_params(q);
     const int K = layer_k(l), N = layer_n(l), kr = real_k(l), nr = real_n(l);
@@ -312,6 +602,7 @@ __global__ void k_adam(AdamArgs a) {
         }
     };
     if (a.apply == 2) {  // pack only: BF16 copies of the current masters
+        if (!have || grp) return;
         if (is_w) {
             k = (int)(t / nr);
             n = (int)(t % nr);
@@ -327,15 +618,28 @@ __global__ void k_adam(AdamArgs a) {
     if (is_w) {
         k = (int)(t / nr);
         n = (int)(t % nr);
-        // the weight-gradient product is [n][k] for the hidden layers and [k][n] for the output layer
-        for (int s = 0; s < a.splits; s++)
-            g += (l < kNHid) ? a.dw[l][((long long)s * kTileRows + n) * dw_cols(l) + k]
-                             : a.dw[l][((long long)s * kTileRows + k) * N + n];
     } else {
         n = (int)(t - (long long)kr * nr);
-        const int stride = (l < kNHid) ? kTileRows : kOut;
-        for (int s = 0; s < a.tiles; s++) g += a.db[l][(long long)s * stride + n];
     }
+    if (have) {
+        if (a.part) {
+            for (int s = grp; s < a.splits; s += kAdamGroup) g += a.part[(long long)s * param_count() + off + t];
+        } else if (is_w) {
+            // the weight-gradient product is [n][k] for the hidden layers and [k][n] for the output layer
+            for (int s = grp; s < a.splits; s += kAdamGroup)
+                g += (l < kNHid) ? a.dw[l][((long long)s * kTileRows + n) * dw_cols(l) + k]
+                                 : a.dw[l][((long long)s * kTileRows + k) * N + n];
+        } else {
+            const int stride = (l < kNHid) ? kTileRows : kOut;
+            for (int s = grp; s < a.tiles; s += kAdamGroup) g += a.db[l][(long long)s * stride + n];
+        }
+    }
+    __shared__ float sums[kAdamGroup][kAdamParams];
+    sums[grp][col] = g;
+    __syncthreads();
+    if (grp || !have) return;
+#pragma unroll
+    for (int q = 1; q < kAdamGroup; q++) g += sums[q][col];
     if (a.gout) a.gout[off + t] = g;
     if (!a.apply) return;
     float *p = is_w ? &a.W[l][k * N + n] : &a.b[l][n];
@@ -429,6 +733,8 @@ struct dg_nn {
     bf16 *Xn = nullptr, *Xt = nullptr, *Hn[kNHid] = {}, *Ht[kNHid] = {}, *Dn[2] = {}, *Dt[2] = {}, *D3n = nullptr,
          *D3t = nullptr;
     float *Tb = nullptr, *Y = nullptr, *G[kNHid] = {}, *dw[kNL] = {}, *db[kNL] = {}, *lpart = nullptr, *gout = nullptr;
+    float *part = nullptr;       // per-block gradients of the one-kernel pass (param_count() each) ...
+    long long lparts = 0;        // ... and the loss sums the last pass left in lpart
     long long step = 0;
     unsigned long long seed = 1;
     float beta1 = 0.9f, beta2 = 0.999f, eps = 1e-8f;
@@ -502,10 +808,15 @@ int ensure_batch(dg_nn *n, long long rows) {
         (rc = scratch_t(n, &n->D3n, R * kOutPad)) || (rc = scratch_t(n, &n->D3t, R * kOutPad)) ||
         (rc = scratch_t(n, &n->lpart, tiles)) || (rc = scratch_t(n, &n->gout, dg_nn_param_count())))
         return rc;
+    if (kTrainFused && (rc = scratch_t(n, &n->part, std::min<long long>(tiles, kTrainBlocks) * param_count()))) return rc;
     for (int l = 0; l < kNHid; l++)
         if ((rc = scratch_t(n, &n->Hn[l], R * kHid)) || (rc = scratch_t(n, &n->Ht[l], R * kHidT)) ||
             (rc = scratch_t(n, &n->G[l], R * kHid)))
             return rc;
+    if (kTrainFused) {  // the kernel chain's gradient operands are not used
+        n->bcap = rows;
+        return 0;
+    }
     for (int q = 0; q < 2; q++)
         if ((rc = scratch_t(n, &n->Dn[q], R * kHid)) || (rc = scratch_t(n, &n->Dt[q], R * kHidT))) return rc;
     for (int l = 0; l < kNL; l++)
@@ -551,7 +862,9 @@ int forward(dg_nn *n, long long rows) {
     return launch_gemm<M_FWD_OUT, kOutPad>(n, g, tiles);
 }
 
-// loss gradient and backward pass; leaves weight/bias gradient partials in dw/db
+// loss gradient and backward pass; leaves weight/bias gradient partials in dw/db (a template: the
+// kernels of the chain are built only for the shapes that use it)
+template <int = 0>
 int backward(dg_nn *n, long long rows, long long valid) {
     const long long tiles = rows / kTileRows;
     const int csplit = (rows % 512 == 0) ? 512 : 128;
@@ -587,6 +900,9 @@ int backward(dg_nn *n, long long rows, long long valid) {
     return 0;
 }
 
+// blocks of the one-kernel pass: one per SM (its tensor memory)
+int train_blocks(long long rows) { return (int)std::min<long long>(rows / kTileRows, kTrainBlocks); }
+
 int adam(dg_nn *n, long long rows, float lr, int apply, float *gout) {
     AdamArgs a{};
     for (int l = 0; l < kNL; l++) {
@@ -596,6 +912,10 @@ int adam(dg_nn *n, long long rows, float lr, int apply, float *gout) {
     }
     a.splits = (int)(rows / ((rows % 512 == 0) ? 512 : 128));
     a.tiles = (int)(rows / kTileRows);
+    if (kTrainFused) {
+        a.part = n->part;
+        a.splits = train_blocks(rows);
+    }
     a.lr = lr; a.beta1 = n->beta1; a.beta2 = n->beta2; a.eps = n->eps;
     if (apply == 1) n->step++;
     const double t = (double)(n->step > 0 ? n->step : 1);
@@ -604,7 +924,7 @@ int adam(dg_nn *n, long long rows, float lr, int apply, float *gout) {
     a.apply = apply;
     a.gout = gout;
     const long long np = dg_nn_param_count();
-    k_adam<<<(unsigned)((np + 255) / 256), 256, 0, n->stream>>>(a);
+    k_adam<<<(unsigned)((np + kAdamParams - 1) / kAdamParams), kAdamGroup * kAdamParams, 0, n->stream>>>(a);
     NN_CUDA(cudaGetLastError());
     return 0;
 }
@@ -615,6 +935,28 @@ int gather(dg_nn *n, long long rows, int random, long long first) {
                                                                       first, n->d_sc, n->Xn, n->Xt, n->Tb);
     NN_CUDA(cudaGetLastError());
     return 0;
+}
+
+// gradient and loss sums of one batch (rows drawn at random, or in order from the first sample)
+int gradient_pass(dg_nn *n, long long rows, int random) {
+    if constexpr (kTrainFused) {
+        TrainArgs g{};
+        g.xs = n->xs; g.ts = n->ts; g.ns = n->ns; g.rows = rows; g.first = 0; g.random = random;
+        g.seed = n->seed + 0x9E37ull * (unsigned long long)n->step;
+        g.sc = n->d_sc;
+        for (int l = 0; l < kNL; l++) { g.Wt[l] = n->Wt[l]; g.Wn[l] = n->Wn[l]; g.b[l] = n->b[l]; }
+        g.part = n->part; g.lpart = n->lpart; g.err = n->d_err;
+        n->lparts = train_blocks(rows);
+        NN_CUDA(cudaFuncSetAttribute(k_train, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrainSmem));
+        k_train<<<(unsigned)n->lparts, kTrainThreads, kTrainSmem, n->stream>>>(g);
+        NN_CUDA(cudaGetLastError());
+        return 0;
+    } else {
+        int rc;
+        n->lparts = rows / kTileRows;
+        if ((rc = gather(n, rows, random, 0)) || (rc = forward(n, rows))) return rc;
+        return backward<>(n, rows, rows);
+    }
 }
 
 // write the BF16 operand copies of the FP32 masters
@@ -809,12 +1151,10 @@ int dg_nn_train(dg_nn *n, int steps, int batch, float lr, float *loss_out) {
     NN_CUDA(cudaSetDevice(n->device));
     if ((rc = ensure_batch(n, batch))) return rc;
     for (int s = 0; s < steps; s++) {
-        if ((rc = gather(n, batch, 1, 0)) || (rc = forward(n, batch)) || (rc = backward(n, batch, batch)) ||
-            (rc = adam(n, batch, lr, 1, nullptr)))
-            return rc;
+        if ((rc = gradient_pass(n, batch, 1)) || (rc = adam(n, batch, lr, 1, nullptr))) return rc;
     }
     if (loss_out) {
-        std::vector<float> lp((size_t)batch / kTileRows);
+        std::vector<float> lp((size_t)n->lparts);
         NN_CUDA(cudaMemcpyAsync(lp.data(), n->lpart, lp.size() * sizeof(float), cudaMemcpyDeviceToHost, n->stream));
         if ((rc = nn_sync(n))) return rc;
         double l = 0.0;
@@ -836,14 +1176,12 @@ int dg_nn_gradients(dg_nn *n, const float *x, const float *t, int batch, float *
     const long long ns = n->ns, cap = n->cap;
     n->xs = nullptr; n->ts = nullptr; n->ns = 0; n->cap = 0;
     rc = dg_nn_set_samples(n, x, t, batch);
-    if (!rc) rc = gather(n, batch, 0, 0);
-    if (!rc) rc = forward(n, batch);
-    if (!rc) rc = backward(n, batch, batch);
+    if (!rc) rc = gradient_pass(n, batch, 0);
     if (!rc) rc = adam(n, batch, 0.0f, 0, n->gout);
     const long long np = dg_nn_param_count();
     if (!rc && cudaMemcpyAsync(grad, n->gout, (size_t)np * sizeof(float), cudaMemcpyDeviceToHost, n->stream) != cudaSuccess)
         rc = nn_fail(DG_ERR_CUDA, "gradient read-back failed");
-    std::vector<float> lp((size_t)batch / kTileRows);
+    std::vector<float> lp((size_t)(rc ? 0 : n->lparts));
     if (!rc && cudaMemcpyAsync(lp.data(), n->lpart, lp.size() * sizeof(float), cudaMemcpyDeviceToHost, n->stream) != cudaSuccess)
         rc = nn_fail(DG_ERR_CUDA, "loss read-back failed");
     if (!rc) rc = nn_sync(n);
