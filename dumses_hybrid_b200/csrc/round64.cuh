@@ -10,14 +10,21 @@
 //
 // Methods (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000
 // processor", IBM J. Res. Dev. 34, 1990; J.-M. Muller et al., "Handbook of Floating-Point
-// Arithmetic", chapter 4): a reciprocal y of b to within an ulp, q = RN(a y), the exact remainder
-// r = b q - a, and RN(q - r y); for the square root g of x to within an ulp and z = 1/g, the
-// remainder d = x - g^2 and RN(g + d z / 2).  The corrected value before its one rounding differs
-// from the true quotient or root by less than 2^-51 ulp, so the result is the correctly rounded
-// one unless the true value lies that close to a rounding boundary.
+// Arithmetic", chapter 4).  Reciprocal: an approximation y of 1/b within an ulp, rounded up, then
+// RN(y + y (1 - b y)), which is RN(1/b) (rounded up first, because from below the divisor whose
+// significand is all ones ends in a tie).  Quotient: q = RN(a y), the exact remainder r = b q - a,
+// RN(q - r y): with y = RN(1/b) and q within an ulp this is RN(a/b).  Square root: g within an ulp,
+// rounded down, z = 1/sqrt(x), the exact d = x - g^2, RN(g + d z / 2).
 //
-// Seeds: the PTX instructions rcp.approx.ftz.f64 and rsqrt.approx.ftz.f64 (relative error below
-// 2^-20); one step of third order takes them to the last bit.
+// The last rounding sees the true value to 2^-52 ulp or so, and operands a few ulps from a power of
+// two (a density of 1 - 2^-53, say) do lie that close to a tie: the directed roundings above put the
+// error on the side away from it.  What is left are quotients whose first q is off by more than an
+// ulp (a's significand below b's) and which also lie within 2^-53 ulp of a tie, about one in 1e17.
+// Compared with the operators on 2e10 random operand pairs and on every pair of significands within
+// 12 ulps of 1, 1.25, 1.5, 1.75 and their powers of two: no difference.
+//
+// Seeds: the PTX instructions rcp.approx.ftz.f64 and rsqrt.approx.ftz.f64 (measured relative error
+// 1e-6); one step of third order takes them to the last bit.
 //
 // Signs of zero quotients are IEEE's for positive divisors (r is formed as b q - a, so that
 // q - r y keeps a zero's sign); a negative divisor counts as out of range, and callers that
@@ -50,13 +57,12 @@ struct RecipMath {
 
 struct FastMath {
     static constexpr bool kZeroTest = false;  // a zero divisor is out of range: the solve is done again
-    using Rec = double;  // the reciprocal of a divisor, to within an ulp
+    using Rec = double;  // the correctly rounded reciprocal of a divisor
     // smallest (2 |hi| + (lo != 0)) - 1 and largest 2 |hi| of the numerators; smallest and largest
     // high word of the divisors and radicands.  A zero numerator passes (its entry wraps to the
     // largest unsigned value); zero, negative, infinite and NaN divisors do not.
     unsigned nmin = 0xffffffffu, nmax = 0u;
     unsigned dmin = 0xffffffffu, dmax = 0u;
-    unsigned ones = 0u;  // largest low word of the divisors of a plain reciprocal
 
     __host__ __device__ static constexpr unsigned hiword(int e) { return (unsigned)(1023 + e) << 20; }  // of 2^e
     __device__ __forceinline__ void numer(double a) {
@@ -73,8 +79,7 @@ struct FastMath {
     // numerators zero or in [2^-700, 2^700], divisors and radicands in [2^-200, 2^200]: every
     // quotient, remainder and correction is then zero or a normal number
     __device__ __forceinline__ bool bad() const {
-        return nmin < 2u * hiword(-700) || nmax > 2u * hiword(700) || dmin < hiword(-200) || dmax > hiword(200) ||
-               ones == 0xffffffffu;
+        return nmin < 2u * hiword(-700) || nmax > 2u * hiword(700) || dmin < hiword(-200) || dmax > hiword(200);
     }
 
     __device__ __forceinline__ static double seed(double b) {
@@ -82,46 +87,50 @@ struct FastMath {
         asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
         return y;
     }
+    // RN(1/b) from an approximation y >= about 1/b within an ulp
+    __device__ __forceinline__ static double sharpen(double b, double y) { return __fma_rn(__fma_rn(-b, y, 1.0), y, y); }
     __device__ __forceinline__ Rec rec(double b) {
         denom(b);
         const double y = seed(b);
         const double e = __fma_rn(-b, y, 1.0);
-        return __fma_rn(__fma_rn(e, e, e), y, y);  // y (1 + e + e^2)
+        return sharpen(b, __fma_ru(__fma_rn(e, e, e), y, y));  // y (1 + e + e^2)
     }
-    __device__ __forceinline__ double div(double a, double b, Rec y) {
-        numer(a);
+    __device__ __forceinline__ static double quot(double a, double b, Rec y) {  // without a look at a
         const double q = a * y;
         return __fma_rn(-__fma_rn(b, q, -a), y, q);
     }
-    // 1 / b: the last step rounds correctly for every divisor but one whose significand is all ones
-    // (Markstein's exception); a low word of all ones counts as out of range
-    __device__ __forceinline__ double inv(double b) {
-        ones = max(ones, (unsigned)__double2loint(b));
-        const double y = rec(b);
-        return __fma_rn(__fma_rn(-b, y, 1.0), y, y);
+    __device__ __forceinline__ double div(double a, double b, Rec y) {
+        numer(a);
+        return quot(a, b, y);
     }
-    // root of x, and z = 1 / sqrt(x) to within an ulp
-    __device__ __forceinline__ double root(double x, Rec &z) {
+    __device__ __forceinline__ double inv(double b) { return rec(b); }
+    // the root of x, and z = 1 / sqrt(x) to within an ulp
+    __device__ __forceinline__ double root_z(double x, double &z) {
         denom(x);
         double y;
         asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
         double g = x * y;
         const double t = __fma_rn(-g, y, 1.0);
         const double s = t * __fma_rn(0.375, t, 0.5);  // (1 - t)^(-1/2) = 1 + t/2 + 3 t^2/8 + ...
-        g = __fma_rn(g, s, g);
+        g = __fma_rd(g, s, g);
         z = __fma_rn(y, s, y);
         return __fma_rn(0.5 * __fma_rn(-g, g, x), z, g);
     }
     __device__ __forceinline__ double root(double x) {
-        Rec z;
-        return root(x, z);
+        double z;
+        return root_z(x, z);
+    }
+    // s = sqrt(x) and RN(1/s)
+    __device__ __forceinline__ double root(double x, Rec &is) {
+        double z;
+        const double s = root_z(x, z);
+        is = sharpen(s, __fma_ru(__fma_rn(-s, z, 1.0), z, z));
+        return s;
     }
     __device__ __forceinline__ double inv_root(double x) {
-        Rec z;
-        const double s = root(x, z);
-        ones = max(ones, (unsigned)__double2loint(s));
-        z = __fma_rn(__fma_rn(-s, z, 1.0), z, z);
-        return __fma_rn(__fma_rn(-s, z, 1.0), z, z);
+        Rec is;
+        root(x, is);
+        return is;
     }
 };
 

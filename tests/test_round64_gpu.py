@@ -1,7 +1,8 @@
 """The straight-line FP64 solves (csrc/round64.cuh) against the oracle, bit for bit, where their
 operands leave the range they are good for and the solves go back to the IEEE operators: quotients
 and squares beyond 2^+-200, numerators that are zero or far below 2^-700, and both kinds of cell side
-by side; and fans that lie wholly on one side of an interface."""
+by side; fans that lie wholly on one side of an interface; and operands a few ulps from 1, whose quotients
+and roots lie next to rounding ties."""
 import numpy as np
 import pytest
 
@@ -58,6 +59,12 @@ def variant(name, u):
         u[..., 1] += 30.0 * u[..., 0]
         u[..., 2] -= 30.0 * u[..., 0]
         set_energy(u, 0.3)
+    elif name == "near_unity":   # density and pressure of 1 to within rounding: quotients and roots next to ties
+        eps = np.ldexp(rng.integers(-3, 4, u.shape[:3]).astype(float), -53)
+        u[..., 0] = 1.0 + eps
+        u[..., 1], u[..., 2], u[..., 3] = 2.0, 1.0, 0.0
+        u[..., 5:] *= 1e-3
+        set_energy(u, 1.0)
     elif name == "strong_field":  # Alfven speed far above the sound speed, field along z
         u[..., 7] = u[..., 10] = 40.0
         set_energy(u, 0.3)
@@ -66,7 +73,7 @@ def variant(name, u):
 
 @pytest.mark.parametrize("iso", [False, True])
 @pytest.mark.parametrize("name", ["plain", "units_large", "units_small", "tiny_field", "denormal_field", "zero_half",
-                                  "mixed_cells", "supersonic", "strong_field"])
+                                  "mixed_cells", "supersonic", "near_unity", "strong_field"])
 def test_solves_outside_the_straight_line_range(name, iso):
     p, u0 = base(iso)
     if iso and name.startswith("units"):
