@@ -135,6 +135,13 @@ double sync_timeout_s() {
     return 300.0;
 }
 
+// Pause between two polls of a wait that began el seconds ago: none for the first 2 ms (a sleep of
+// any length takes about 55 us, the timer's slack, which a short call would wait for nothing: a
+// driver's compute_dt on 32 x 64 x 32 cells 67 us with sleeps), short ones then.
+void poll_pause(double el) {
+    if (el > 0.002) std::this_thread::sleep_for(std::chrono::microseconds(el < 0.01 ? 5 : 100));
+}
+
 // wait for the stream with a wall-clock bound instead of blocking forever
 int bounded_sync(cudaStream_t s) {
     const double limit = sync_timeout_s();
@@ -145,7 +152,7 @@ int bounded_sync(cudaStream_t s) {
         if (e != cudaErrorNotReady) return fail(DG_ERR_CUDA, std::string("stream: ") + cudaGetErrorString(e));
         double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
         if (el > limit) return fail(DG_ERR_TIMEOUT, "device work did not finish within DG_SYNC_TIMEOUT_S");
-        std::this_thread::sleep_for(std::chrono::microseconds(el < 0.01 ? 5 : 200));
+        poll_pause(el);
     }
 }
 
@@ -159,7 +166,7 @@ int bounded_event(cudaEvent_t ev) {
         if (e != cudaErrorNotReady) return fail(DG_ERR_CUDA, std::string("event: ") + cudaGetErrorString(e));
         double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
         if (el > limit) return fail(DG_ERR_TIMEOUT, "device work did not finish within DG_SYNC_TIMEOUT_S");
-        std::this_thread::sleep_for(std::chrono::microseconds(el < 0.01 ? 5 : 200));
+        poll_pause(el);
     }
 }
 

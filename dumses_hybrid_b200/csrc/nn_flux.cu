@@ -723,11 +723,14 @@ using namespace dg::nn;
 struct dg_nn {
     int device = 0;
     cudaStream_t stream = nullptr;
-    int *d_err = nullptr;
+    int *d_err = nullptr, *h_err = nullptr;  // device error word and its pinned read-back
     float *W[kNL] = {}, *b[kNL] = {}, *mW[kNL] = {}, *vW[kNL] = {}, *mb[kNL] = {}, *vb[kNL] = {};
     bf16 *Wt[kNL] = {}, *Wn[kNL] = {}, *Bt[kNHid] = {};
     float *xs = nullptr, *ts = nullptr;  // samples
     long long ns = 0, cap = 0;
+    float *gx = nullptr, *gt = nullptr;  // a caller's batch of dg_nn_gradients (gcap rows, kept between calls)
+    float *gh = nullptr;                 // pinned read-back of its gradient and loss sums
+    long long gcap = 0;
     // batch scratch
     long long bcap = 0;
     bf16 *Xn = nullptr, *Xt = nullptr, *Hn[kNHid] = {}, *Ht[kNHid] = {}, *Dn[2] = {}, *Dt[2] = {}, *D3n = nullptr,
@@ -772,14 +775,15 @@ int nn_bounded_sync(cudaStream_t st) {
         if (q != cudaErrorNotReady) return nn_fail(DG_ERR_CUDA, std::string("stream: ") + cudaGetErrorString(q));
         const double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
         if (el > limit) return nn_fail(DG_ERR_TIMEOUT, "device work did not finish within DG_SYNC_TIMEOUT_S");
-        std::this_thread::sleep_for(std::chrono::microseconds(el < 0.01 ? 5 : 200));
+        if (el > 0.002)  // poll without a sleep at first: a sleep of any length takes about 55 us
+            std::this_thread::sleep_for(std::chrono::microseconds(el < 0.01 ? 5 : 100));
     }
 }
 
 int nn_sync(dg_nn *n) {
+    NN_CUDA(cudaMemcpyAsync(n->h_err, n->d_err, sizeof(int), cudaMemcpyDeviceToHost, n->stream));
     if (int rc = nn_bounded_sync(n->stream)) return rc;
-    int err = 0;
-    NN_CUDA(cudaMemcpy(&err, n->d_err, sizeof(int), cudaMemcpyDeviceToHost));
+    const int err = *n->h_err;
     if (err) return nn_fail(DG_ERR_STATE, "network kernel gave up waiting on a tensor-core transfer (error bits " +
                                               std::to_string(err) + ")");
     return 0;
@@ -1042,6 +1046,7 @@ int dg_nn_create(int device, unsigned long long seed, dg_nn **out) {
     if (cudaStreamCreateWithFlags(&n->stream, cudaStreamNonBlocking) != cudaSuccess)
         return bail(nn_fail(DG_ERR_CUDA, "stream creation failed"));
     if ((rc = nn_alloc_t(n, &n->d_err, 1))) return bail(rc);
+    if (cudaMallocHost((void **)&n->h_err, sizeof(int)) != cudaSuccess) return bail(nn_fail(DG_ERR_NOMEM, "cudaMallocHost failed"));
     // He-normal initial weights on the host from the seed (Box-Muller over splitmix64)
     unsigned long long st = seed * 0x9E3779B97F4A7C15ull + 12345u;
     auto next = [&]() {
@@ -1093,6 +1098,10 @@ int dg_nn_destroy(dg_nn *n) {
     for (void *p : n->scratch) cudaFree(p);
     if (n->xs) cudaFree(n->xs);
     if (n->ts) cudaFree(n->ts);
+    if (n->gx) cudaFree(n->gx);
+    if (n->gt) cudaFree(n->gt);
+    if (n->gh) cudaFreeHost(n->gh);
+    if (n->h_err) cudaFreeHost(n->h_err);
     if (n->stream) cudaStreamDestroy(n->stream);
     delete n;
     return DG_OK;
@@ -1171,29 +1180,46 @@ int dg_nn_gradients(dg_nn *n, const float *x, const float *t, int batch, float *
     if ((rc = check_batch(batch))) return rc;
     NN_CUDA(cudaSetDevice(n->device));
     if ((rc = ensure_batch(n, batch))) return rc;
-    // a private sample set holding exactly this batch, in order
+    // a private sample set holding exactly this batch, in order, in buffers kept for the next call
+    // (allocating and freeing them was two thirds of a call on 16384 rows)
+    const long long np = dg_nn_param_count(), nl = batch / kTileRows;
+    if (batch > n->gcap) {
+        NN_CUDA(cudaStreamSynchronize(n->stream));
+        if (n->gx) cudaFree(n->gx);
+        if (n->gt) cudaFree(n->gt);
+        if (n->gh) cudaFreeHost(n->gh);
+        n->gx = n->gt = n->gh = nullptr;
+        n->gcap = 0;
+        if (cudaMalloc(&n->gx, (size_t)batch * kIn * sizeof(float)) != cudaSuccess ||
+            cudaMalloc(&n->gt, (size_t)batch * kOut * sizeof(float)) != cudaSuccess ||
+            cudaMallocHost(&n->gh, (size_t)(np + nl) * sizeof(float)) != cudaSuccess) {
+            cudaGetLastError();
+            return nn_fail(DG_ERR_CUDA, "out of memory for the gradient batch");
+        }
+        n->gcap = batch;
+    }
+    NN_CUDA(cudaMemcpyAsync(n->gx, x, (size_t)batch * kIn * sizeof(float), cudaMemcpyHostToDevice, n->stream));
+    NN_CUDA(cudaMemcpyAsync(n->gt, t, (size_t)batch * kOut * sizeof(float), cudaMemcpyHostToDevice, n->stream));
     float *xs = n->xs, *ts = n->ts;
-    const long long ns = n->ns, cap = n->cap;
-    n->xs = nullptr; n->ts = nullptr; n->ns = 0; n->cap = 0;
-    rc = dg_nn_set_samples(n, x, t, batch);
-    if (!rc) rc = gradient_pass(n, batch, 0);
+    const long long ns = n->ns;
+    n->xs = n->gx; n->ts = n->gt; n->ns = batch;
+    rc = gradient_pass(n, batch, 0);
     if (!rc) rc = adam(n, batch, 0.0f, 0, n->gout);
-    const long long np = dg_nn_param_count();
-    if (!rc && cudaMemcpyAsync(grad, n->gout, (size_t)np * sizeof(float), cudaMemcpyDeviceToHost, n->stream) != cudaSuccess)
-        rc = nn_fail(DG_ERR_CUDA, "gradient read-back failed");
-    std::vector<float> lp((size_t)(rc ? 0 : n->lparts));
-    if (!rc && cudaMemcpyAsync(lp.data(), n->lpart, lp.size() * sizeof(float), cudaMemcpyDeviceToHost, n->stream) != cudaSuccess)
-        rc = nn_fail(DG_ERR_CUDA, "loss read-back failed");
-    if (!rc) rc = nn_sync(n);
-    if (n->xs) cudaFree(n->xs);
-    if (n->ts) cudaFree(n->ts);
-    n->xs = xs; n->ts = ts; n->ns = ns; n->cap = cap;
-    if (!rc && loss) {
+    n->xs = xs; n->ts = ts; n->ns = ns;
+    if (rc) {
+        nn_bounded_sync(n->stream);
+        return rc;
+    }
+    NN_CUDA(cudaMemcpyAsync(n->gh, n->gout, (size_t)np * sizeof(float), cudaMemcpyDeviceToHost, n->stream));
+    NN_CUDA(cudaMemcpyAsync(n->gh + np, n->lpart, (size_t)n->lparts * sizeof(float), cudaMemcpyDeviceToHost, n->stream));
+    if ((rc = nn_sync(n))) return rc;
+    std::memcpy(grad, n->gh, (size_t)np * sizeof(float));
+    if (loss) {
         double l = 0.0;
-        for (float v : lp) l += v;
+        for (long long q = 0; q < n->lparts; q++) l += n->gh[np + q];
         *loss = (float)(l / ((double)batch * kOut));
     }
-    return rc;
+    return DG_OK;
 }
 
 int dg_nn_forward(dg_nn *n, const float *x, long long count, float *y) {
