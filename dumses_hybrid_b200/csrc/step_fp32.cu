@@ -331,10 +331,11 @@ __device__ __forceinline__ float slope_hl(int ist, HL m, HL c, HL p) {
 }
 // emfx (i in 1..nx, k in 1..nz+1) and emfz (i in 1..nx+1, k in 1..nz) over j in 1..ny+1,
 // along y lines as the FP64 kernel does (shift once per column, sliding donor window)
+template <int SEG>
 __global__ void __launch_bounds__(kThreads) k_fargo_emf_hl(Geo G, StoreHL U, float *__restrict__ fex,
                                                            float *__restrict__ fez, const Scalars *S) {
     FargoLine L;
-    if (!fargo_line(G, blockIdx.x * (long long)blockDim.x + threadIdx.x, L)) return;
+    if (!fargo_line(G, blockIdx.x * (long long)blockDim.x + threadIdx.x, SEG, L)) return;
     const int i = L.i, k = L.k;
     const double dt = S->dt;
     const float dy = (float)G.dy;
@@ -388,11 +389,12 @@ __global__ void __launch_bounds__(kThreads) k_fargo_emf_hl(Geo G, StoreHL U, flo
 #ifndef DG_FARGO_MINB32
 #define DG_FARGO_MINB32 3
 #endif
+template <int SEG>
 __global__ void __launch_bounds__(kThreads, DG_FARGO_MINB32) k_fargo_update_hl(Geo G, StoreHL U, StoreHL Un,
                                                               const float *__restrict__ fex,
                                                               const float *__restrict__ fez, const Scalars *S) {
     FargoLine L;
-    if (!fargo_line(G, blockIdx.x * (long long)blockDim.x + threadIdx.x, L)) return;
+    if (!fargo_line(G, blockIdx.x * (long long)blockDim.x + threadIdx.x, SEG, L)) return;
     const int i = L.i, k = L.k;
     const int nx = G.nx, ny = G.ny, nz = G.nz;
     if (i <= nx && k <= nz && L.jb <= ny) {
@@ -405,17 +407,17 @@ __global__ void __launch_bounds__(kThreads, DG_FARGO_MINB32) k_fargo_update_hl(G
         const int js = fargo_src(f, L.jb, ny);
         const int j0 = js - 1 < 1 ? js - 1 + ny : js - 1;  // the window starts one row below the first donor
         for (int v = IR; v <= IP; v++) {
-            // rows js-1 .. js+kFargoSeg+1 (periodic y); rows past the segment's end are loaded but unused
-            HL wn[kFargoSeg + 3];
+            // rows js-1 .. js+SEG+1 (periodic y); rows past the segment's end are loaded but unused
+            HL wn[SEG + 3];
             int row = j0;
 #pragma unroll
-            for (int m = 0; m < kFargoSeg + 3; m++) {
+            for (int m = 0; m < SEG + 3; m++) {
                 wn[m] = hl_at(G, U, v, G.idx(i, row, k));
                 row = next_row(row, ny);
             }
             float s0 = slope_hl(ist, wn[0], wn[1], wn[2]);
 #pragma unroll
-            for (int m = 0; m < kFargoSeg; m++) {
+            for (int m = 0; m < SEG; m++) {
                 const int j = L.jb + m;
                 if (j > L.je || j > ny) break;
                 const float s1 = slope_hl(ist, wn[m + 1], wn[m + 2], wn[m + 3]);
@@ -951,8 +953,12 @@ int launch_harvest(const Geo &G, const Bufs &B, int d, int stride, float *xs, fl
 
 int launch_fargo(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
     float *fex = (float *)B.femf[0], *fez = (float *)B.femf[1];
-    TIMED(KS_FARGO_EMF, s, (k_fargo_emf_hl<<<nblocks(fargo_line_threads(G), kThreads), kThreads, 0, s>>>(G, st(B, cur), fex, fez, B.S)));
-    TIMED(KS_FARGO_UPDATE, s, (k_fargo_update_hl<<<nblocks(fargo_line_threads(G), kThreads), kThreads, 0, s>>>(G, st(B, cur), st(B, cur ^ 1), fex, fez, B.S)));
+    const StoreHL U = st(B, cur), Un = st(B, cur ^ 1);
+    const unsigned nl = nblocks(fargo_line_threads(G, kFargoLong), kThreads), ns = nblocks(fargo_line_threads(G, kFargoShort), kThreads);
+    if (fargo_short(G, 2.0)) TIMED(KS_FARGO_EMF, s, (k_fargo_emf_hl<kFargoShort><<<ns, kThreads, 0, s>>>(G, U, fex, fez, B.S)));
+    else TIMED(KS_FARGO_EMF, s, (k_fargo_emf_hl<kFargoLong><<<nl, kThreads, 0, s>>>(G, U, fex, fez, B.S)));
+    if (fargo_short(G, 0.75)) TIMED(KS_FARGO_UPDATE, s, (k_fargo_update_hl<kFargoShort><<<ns, kThreads, 0, s>>>(G, U, Un, fex, fez, B.S)));
+    else TIMED(KS_FARGO_UPDATE, s, (k_fargo_update_hl<kFargoLong><<<nl, kThreads, 0, s>>>(G, U, Un, fex, fez, B.S)));
     return 2;
 }
 

@@ -373,8 +373,12 @@ int launch_godunov(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
 }
 
 int launch_fargo(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
-    TIMED(KS_FARGO_EMF, s, (k_fargo_emf<StoreD><<<nblocks(fargo_line_threads(G), kThreads), kThreads, 0, s>>>(G, st(B, cur), B.femf[0], B.femf[1], B.S)));
-    TIMED(KS_FARGO_UPDATE, s, (k_fargo_update<StoreD><<<nblocks(fargo_line_threads(G), kThreads), kThreads, 0, s>>>(G, st(B, cur), st(B, cur ^ 1), B.femf[0], B.femf[1], B.S)));
+    const StoreD U = st(B, cur), Un = st(B, cur ^ 1);
+    const unsigned nl = nblocks(fargo_line_threads(G, kFargoLong), kThreads), ns = nblocks(fargo_line_threads(G, kFargoShort), kThreads);
+    if (fargo_short(G, 2.0)) TIMED(KS_FARGO_EMF, s, (k_fargo_emf<StoreD, kFargoShort><<<ns, kThreads, 0, s>>>(G, U, B.femf[0], B.femf[1], B.S)));
+    else TIMED(KS_FARGO_EMF, s, (k_fargo_emf<StoreD, kFargoLong><<<nl, kThreads, 0, s>>>(G, U, B.femf[0], B.femf[1], B.S)));
+    if (fargo_short(G, 0.75)) TIMED(KS_FARGO_UPDATE, s, (k_fargo_update<StoreD, kFargoShort><<<ns, kThreads, 0, s>>>(G, U, Un, B.femf[0], B.femf[1], B.S)));
+    else TIMED(KS_FARGO_UPDATE, s, (k_fargo_update<StoreD, kFargoLong><<<nl, kThreads, 0, s>>>(G, U, Un, B.femf[0], B.femf[1], B.S)));
     return 2;
 }
 

@@ -1924,29 +1924,32 @@ __device__ __forceinline__ double fslope(const Geo &G, const Store &U, int v, in
     return limit1<double>((double)st, val(j - 1), val(j), val(j + 1));
 }
 
-// FARGO line layout: one thread per (i, k) face column and per segment of kFargoSeg faces
-// along y; consecutive threads take consecutive i (coalesced), and a thread slides a
-// window of source values along its segment so each source value is read once
-#ifndef DG_FARGO_SEG
-#define DG_FARGO_SEG 16
-#endif
-constexpr int kFargoSeg = DG_FARGO_SEG;
+// FARGO line layout: one thread per (i, k) face column and per segment of SEG faces along y;
+// consecutive threads take consecutive i (coalesced), and a thread slides a window of source values
+// along its segment (or, for the remap, loads the whole window at once), so each source value is
+// read once.  Segments of 16 rows read 1.2 values per row, segments of 4 1.75, but they are a quarter
+// as long a chain and four times the threads.  They are taken where 16-row segments fill less than
+// so many waves of blocks: 2 for the EMFs (90 x 126 x 70 cells, 0.9 wave: 35 -> 21 us), 3/4 for the
+// remap (there 37 -> 41 us; 64^3, 0.4 wave: 23 -> 17 us in FP32).  32 x 64 x 32 cells, FP64: EMFs 29 ->
+// 13 us, remap 29 -> 15 us.
+constexpr int kFargoLong = 16, kFargoShort = 4;
 constexpr int kFargoChunk = 4;  // rows of the CT part whose loads are issued together
-__host__ __device__ __forceinline__ long long fargo_line_threads(const Geo &G) {
-    return (long long)G.FX * G.FZ * ((G.FY + kFargoSeg - 1) / kFargoSeg);
+__host__ __device__ __forceinline__ long long fargo_line_threads(const Geo &G, int seg) {
+    return (long long)G.FX * G.FZ * ((G.FY + seg - 1) / seg);
 }
+inline bool fargo_short(const Geo &G, double waves) { return fargo_line_threads(G, kFargoLong) < waves * 148 * 3 * kThreads; }
 struct FargoLine {
     int i, k, jb, je;  // face column and the segment [jb, je] of y faces
 };
-__device__ __forceinline__ bool fargo_line(const Geo &G, long long t, FargoLine &L) {
-    const int nseg = (G.FY + kFargoSeg - 1) / kFargoSeg;
+__device__ __forceinline__ bool fargo_line(const Geo &G, long long t, int seg, FargoLine &L) {
+    const int nseg = (G.FY + seg - 1) / seg;
     if (t >= 2147483647LL) return false;
     int sg;
     split3((unsigned)t, G.dFX, G.dFZ, L.i, L.k, sg);
     L.i++; L.k++;
     if (sg >= nseg) return false;
-    L.jb = (int)sg * kFargoSeg + 1;
-    L.je = mn(L.jb + kFargoSeg - 1, G.FY);
+    L.jb = (int)sg * seg + 1;
+    L.je = mn(L.jb + seg - 1, G.FY);
     return true;
 }
 // donor row js of row j for the column's shift, fargo.f90:63-77
@@ -1975,11 +1978,11 @@ __device__ __forceinline__ int fargo_zplane(const Geo &G, int k) {
 // emfx (i in 1..nx, k in 1..nz+1) and emfz (i in 1..nx+1, k in 1..nz) over j in 1..ny+1,
 // along y lines (fargo_line): per column the shift is computed once and the donor field and
 // its two neighbours (for uin_slope) slide along the segment
-template <class Store>
+template <class Store, int SEG>
 __global__ void __launch_bounds__(kThreads) k_fargo_emf(Geo G, Store U, double *__restrict__ fex,
                                                         double *__restrict__ fez, const Scalars *S) {
     FargoLine L;
-    if (!fargo_line(G, blockIdx.x * (long long)blockDim.x + threadIdx.x, L)) return;
+    if (!fargo_line(G, blockIdx.x * (long long)blockDim.x + threadIdx.x, SEG, L)) return;
     const int i = L.i, k = L.k;
     const double dt = S->dt, dy = G.dy, half = 0.5, one = 1.0;
     const int ny = G.ny, st = mn(G.slope_type, 2);
@@ -2035,11 +2038,11 @@ __global__ void __launch_bounds__(kThreads) k_fargo_emf(Geo G, Store U, double *
 #ifndef DG_FARGO_MINB64
 #define DG_FARGO_MINB64 3
 #endif
-template <class Store>
+template <class Store, int SEG>
 __global__ void __launch_bounds__(kThreads, DG_FARGO_MINB64) k_fargo_update(Geo G, Store U, Store Un, const double *__restrict__ fex,
                                                            const double *__restrict__ fez, const Scalars *S) {
     FargoLine L;
-    if (!fargo_line(G, blockIdx.x * (long long)blockDim.x + threadIdx.x, L)) return;
+    if (!fargo_line(G, blockIdx.x * (long long)blockDim.x + threadIdx.x, SEG, L)) return;
     const int i = L.i, k = L.k;
     const int nx = G.nx, ny = G.ny, nz = G.nz;
     const double dt = S->dt, half = 0.5, forth = 0.25, one = 1.0;
@@ -2051,17 +2054,17 @@ __global__ void __launch_bounds__(kThreads, DG_FARGO_MINB64) k_fargo_update(Geo 
         const int js = fargo_src(f, L.jb, ny);
         const int j0 = js - 1 < 1 ? js - 1 + ny : js - 1;  // the window starts one row below the first donor
         for (int v = IR; v <= IP; v++) {
-            // rows js-1 .. js+kFargoSeg+1 (periodic y); rows past the segment's end are loaded but unused
-            double wn[kFargoSeg + 3];
+            // rows js-1 .. js+SEG+1 (periodic y); rows past the segment's end are loaded but unused
+            double wn[SEG + 3];
             int row = j0;
 #pragma unroll
-            for (int m = 0; m < kFargoSeg + 3; m++) {
+            for (int m = 0; m < SEG + 3; m++) {
                 wn[m] = U.getr(G, v, G.idx(i, row, k));
                 row = next_row(row, ny);
             }
             double s0 = lim(wn[0], wn[1], wn[2]);
 #pragma unroll
-            for (int m = 0; m < kFargoSeg; m++) {
+            for (int m = 0; m < SEG; m++) {
                 const int j = L.jb + m;
                 if (j > L.je || j > ny) break;
                 const double s1 = lim(wn[m + 1], wn[m + 2], wn[m + 3]);
