@@ -388,10 +388,9 @@ int dg_init(const dg_params *p, dg_ctx **out) {
         if (p->ndim == 1 || (p->ndim == 2 && d < 2)) continue;
         if ((rc = alloc_w(c, &c->B.emf[d], (size_t)G.fsz))) return bail(rc);
     }
-    for (int d = 0; d < 3; d++) {
-        if (p->ndim == 1 || (p->ndim == 2 && d < 2)) continue;
-        if ((rc = alloc_w(c, &c->B.E[d], (size_t)G.esz))) return bail(rc);
-    }
+    // the trace's edge fields as arrays: only the interface harvest of FP32 contexts forms them
+    for (int d = 0; d < 3; d++)
+        if (p->ndim == 3 && p->precision == DG_PREC_FP32 && (rc = alloc_w(c, &c->B.E[d], (size_t)G.esz))) return bail(rc);
     if (p->fargo)
         for (int d = 0; d < 2; d++)
             if ((rc = alloc(c, &c->B.femf[d], (size_t)G.fsz))) return bail(rc);

@@ -48,13 +48,6 @@ struct IeeeMath {
     __device__ __forceinline__ bool bad() const { return false; }
 };
 
-// FP32 quotients as products with the divisor's reciprocal (the mixed path's arithmetic).
-struct RecipMath {
-    using Rec = float;
-    __device__ __forceinline__ Rec rec(float b) { return 1.0f / b; }
-    __device__ __forceinline__ float div(float a, float, Rec y) { return a * y; }
-};
-
 struct FastMath {
     static constexpr bool kZeroTest = false;  // a zero divisor is out of range: the solve is done again
     using Rec = double;  // the correctly rounded reciprocal of a divisor

@@ -850,7 +850,6 @@ constexpr bool kRiemannSplit32 = DG_RIEMANN_SPLIT32 != 0;
 int launch_godunov(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
     const StoreHL U = st(B, cur), Un = st(B, cur ^ 1);
     float *Q = (float *)B.Q, *core = (float *)B.core;
-    float *E2 = (float *)B.E[2];
     float *fx = (float *)B.flx[0], *fy = (float *)B.flx[1], *fz = (float *)B.flx[2];
     float *ex = (float *)B.emf[0], *ey = (float *)B.emf[1], *ez = (float *)B.emf[2];
     const int ni = G.nx + 5, nj = (G.ndim > 1) ? G.ny + 5 : 1, nk = (G.ndim == 3) ? G.nz + 5 : 1;
@@ -867,9 +866,7 @@ int launch_godunov(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
     if (G.ndim == 3) {
         TIMED(KS_TRACE, s, (launch_trace_tile<float, 0>(G, Q, U.hi, core, B.S, s)));
     } else {
-        TIMED(KS_EFIELD, s, (k_efield2d<float><<<nblocks(G.esz, kThreads), kThreads, 0, s>>>(G, Q, U.hi, E2)));
-        TIMED(KS_TRACE, s, (k_trace2d<float><<<nblocks(G.csz, kThreads), kThreads, 0, s>>>(G, Q, U.hi, E2, core, B.S)));
-        n++;
+        TIMED(KS_TRACE, s, (k_trace2d<float><<<nblocks(G.csz, kThreads), kThreads, 0, s>>>(G, Q, U.hi, core, B.S)));
     }
     float *fl[3] = {fx, fy, fz};
     if (B.net) {
@@ -901,7 +898,7 @@ int launch_godunov(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
             TIMED(KS_RIEMANN, s, (k_riemann3d<float, false><<<nb, kThreads, 0, s>>>(G, core, fx, fy, fz, ex, ey, ez, B.S, faces)));
         }
     } else {
-        TIMED(KS_RIEMANN, s, (k_riemann2d<float><<<nblocks(G.fsz, kThreads), kThreads, 0, s>>>(G, core, fx, fy, ez, B.S, faces)));
+        TIMED(KS_RIEMANN, s, (launch_riemann2d<float>(G, core, fx, fy, ez, B.S, faces, s)));
     }
     if (B.net) {
         for (int d = 0; d < G.ndim; d++) {
@@ -930,10 +927,9 @@ int launch_trace_only(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
         TIMED(KS_EFIELD, s, (k_efield3d<float><<<nblocks(G.esz, kThreads), kThreads, 0, s>>>(G, Q, U.hi, E0, E1, E2)));
         TIMED(KS_TRACE, s, (k_trace3d<float><<<nblocks(G.csz, kThreads), kThreads, 0, s>>>(G, Q, U.hi, E0, E1, E2, core, B.S)));
     } else {
-        TIMED(KS_EFIELD, s, (k_efield2d<float><<<nblocks(G.esz, kThreads), kThreads, 0, s>>>(G, Q, U.hi, E2)));
-        TIMED(KS_TRACE, s, (k_trace2d<float><<<nblocks(G.csz, kThreads), kThreads, 0, s>>>(G, Q, U.hi, E2, core, B.S)));
+        TIMED(KS_TRACE, s, (k_trace2d<float><<<nblocks(G.csz, kThreads), kThreads, 0, s>>>(G, Q, U.hi, core, B.S)));
     }
-    return 3 + (G.omega0 > 0.0);
+    return 2 + (G.ndim == 3) + (G.omega0 > 0.0);
 }
 
 const void *nn_faces_kernel() { return (const void *)k_nn_faces; }

@@ -326,7 +326,6 @@ int launch_godunov(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
     const StoreD U = st(B, cur);
     double *Un = (double *)B.U[cur ^ 1];
     double *Q = (double *)B.Q, *core = (double *)B.core;
-    double *E2 = (double *)B.E[2];
     double *fx = (double *)B.flx[0], *fy = (double *)B.flx[1], *fz = (double *)B.flx[2];
     double *ex = (double *)B.emf[0], *ey = (double *)B.emf[1], *ez = (double *)B.emf[2];
     const int ni = G.nx + 5, nj = (G.ndim > 1) ? G.ny + 5 : 1, nk = (G.ndim == 3) ? G.nz + 5 : 1;
@@ -363,11 +362,9 @@ int launch_godunov(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
         else TIMED(KS_RIEMANN, s, (k_riemann1d<double, false><<<nblocks(G.FX, kThreads), kThreads, 0, s>>>(G, core, fx, B.S)));
         TIMED(KS_UPDATE, s, (k_update1d<<<nblocks(G.nx, kThreads), kThreads, 0, s>>>(G, U.p, Un, fx, B.S)));
     } else {
-        TIMED(KS_EFIELD, s, (k_efield2d<double><<<nblocks(G.esz, kThreads), kThreads, 0, s>>>(G, Q, U.p, E2)));
-        TIMED(KS_TRACE, s, (k_trace2d<double><<<nblocks(G.csz, kThreads), kThreads, 0, s>>>(G, Q, U.p, E2, core, B.S)));
-        TIMED(KS_RIEMANN, s, (k_riemann2d<double><<<nblocks(G.fsz, kThreads), kThreads, 0, s>>>(G, core, fx, fy, ez, B.S, 1)));
+        TIMED(KS_TRACE, s, (k_trace2d<double><<<nblocks(G.csz, kThreads), kThreads, 0, s>>>(G, Q, U.p, core, B.S)));
+        TIMED(KS_RIEMANN, s, (launch_riemann2d<double>(G, core, fx, fy, ez, B.S, 1, s)));
         TIMED(KS_UPDATE, s, (k_update2d<<<nblocks(G.fsz, kThreads), kThreads, 0, s>>>(G, U.p, Un, fx, fy, ez, B.S)));
-        n++;
     }
     return n;
 }

@@ -434,6 +434,35 @@ __device__ __forceinline__ T limit1(T st, T qm1, T q0, T qp1) {
     return dsgn * mn(dlim, fab(dcen));
 }
 
+// The quotients x / r of a trace's sources: FP64 takes them from its array of N, divided together by
+// one reciprocal of the density (round64.cuh; by the operator where an operand lies outside its
+// range); FP32 multiplies each by the reciprocal where it is used
+template <typename T, int N>
+struct PerDensity {
+    T n[N], ir;
+    __device__ __forceinline__ PerDensity(const T (&x)[N], T r) {
+        if constexpr (sizeof(T) == 8) {
+            FastMath m;
+            ir = m.rec(r);
+#pragma unroll
+            for (int q = 0; q < N; q++) m.numer(x[q]);
+            if (m.bad()) {
+#pragma unroll
+                for (int q = 0; q < N; q++) n[q] = x[q] / r;
+            } else {
+#pragma unroll
+                for (int q = 0; q < N; q++) n[q] = FastMath::quot(x[q], r, ir);
+            }
+        } else {
+            ir = T(1) / r;
+        }
+    }
+    __device__ __forceinline__ T operator()(int q, T x) const {
+        if constexpr (sizeof(T) == 8) return n[q];
+        else return x * ir;
+    }
+};
+
 // ---------------------------------------------------------------------------
 // edge electric fields and trace
 // ---------------------------------------------------------------------------
@@ -507,17 +536,6 @@ __global__ void __launch_bounds__(kThreads) k_efield3d(Geo G, const T *__restric
     Ex[t] = Ex_at(a, i, j, k);
     Ey[t] = Ey_at(a, i, j, k);
     Ez[t] = Ez_at(a, i, j, k);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kThreads) k_efield2d(Geo G, const T *__restrict__ Q, const T *__restrict__ Bf,
-                                                       T *__restrict__ Ez) {
-    long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= G.esz) return;
-    const int j = (int)fdiv((unsigned)t, G.dEX);
-    const int i = (int)((unsigned)t - (unsigned)j * G.dEX.d);
-    const QV<T> a{Q, Bf, G};
-    Ez[t] = Ez2_at(a, i, j);
 }
 
 template <typename T>
@@ -672,30 +690,11 @@ __device__ __forceinline__ void trace3_cell(const Sten &a, const Geo &G, int i, 
 
     // source terms, scheme.f90:1351-1389
     T sr0 = (-u * drx - dux * r) * dtdx + (-v * dry - dvy * r) * dtdy + (-w * drz - dwz * r) * dtdz;
-    T su0, sv0, sw0;
-    auto velocity_sources = [&](auto &m) {
-        const auto ir = m.rec(r);
-        auto per_r = [&](T x) { return m.div(x, r, ir); };
-        su0 = (-u * dux - per_r(dpx + B * dBx + C * dCx)) * dtdx + (-v * duy + per_r(B * dAy)) * dtdy
-            + (-w * duz + per_r(C * dAz)) * dtdz;
-        sv0 = (-u * dvx + per_r(A * dBx)) * dtdx + (-v * dvy - per_r(dpy + A * dAy + C * dCy)) * dtdy
-            + (-w * dvz + per_r(C * dBz)) * dtdz;
-        sw0 = (-u * dwx + per_r(A * dCx)) * dtdx + (-v * dwy + per_r(B * dCy)) * dtdy
-            + (-w * dwz - per_r(dpz + A * dAz + B * dBz)) * dtdz;
-    };
-    if constexpr (sizeof(T) == 8) {
-        // nine quotients by the density from one reciprocal; again with the operators where an
-        // operand lies outside the range of round64.cuh
-        FastMath m;
-        velocity_sources(m);
-        if (m.bad()) {
-            IeeeMath e;
-            velocity_sources(e);
-        }
-    } else {
-        RecipMath m;
-        velocity_sources(m);
-    }
+    const T gx = dpx + B * dBx + C * dCx, gy = dpy + A * dAy + C * dCy, gz = dpz + A * dAz + B * dBz;
+    const PerDensity<T, 9> d({gx, B * dAy, C * dAz, A * dBx, gy, C * dBz, A * dCx, B * dCy, gz}, r);
+    T su0 = (-u * dux - d(0, gx)) * dtdx + (-v * duy + d(1, B * dAy)) * dtdy + (-w * duz + d(2, C * dAz)) * dtdz;
+    T sv0 = (-u * dvx + d(3, A * dBx)) * dtdx + (-v * dvy - d(4, gy)) * dtdy + (-w * dvz + d(5, C * dBz)) * dtdz;
+    T sw0 = (-u * dwx + d(6, A * dCx)) * dtdx + (-v * dwy + d(7, B * dCy)) * dtdy + (-w * dwz - d(8, gz)) * dtdz;
     T sp0 = (-u * dpx - dux * gamma * p) * dtdx + (-v * dpy - dvy * gamma * p) * dtdy
           + (-w * dpz - dwz * gamma * p) * dtdz;
     T sA0 = (u * dBy + B * duy - v * dAy - A * dvy) * dtdy + (u * dCz + C * duz - w * dAz - A * dwz) * dtdz;
@@ -1069,8 +1068,7 @@ cudaError_t launch_trace_tile(const Geo &G, const T *Q, const T *Bf, T *core, co
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads) k_trace2d(Geo G, const T *__restrict__ Q, const T *__restrict__ Bf,
-                                                      const T *__restrict__ Eza, T *__restrict__ core,
-                                                      const Scalars *S) {
+                                                      T *__restrict__ core, const Scalars *S) {
     long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= G.csz) return;
     const int j = (int)fdiv((unsigned)t, G.dCX);
@@ -1085,8 +1083,9 @@ __global__ void __launch_bounds__(kThreads) k_trace2d(Geo G, const T *__restrict
     const T p = a.q(IP, i, j, k), A = a.q(IA, i, j, k), B = a.q(IB, i, j, k), C = a.q(IC, i, j, k);
     const T AL = a.bf(0, i, j, k), AR = a.bf(0, i + 1, j, k);
     const T BL = a.bf(1, i, j, k), BR = a.bf(1, i, j + 1, k);
-    const T ELL = ld(Eza + G.eidx(i, j, 1)), ELR = ld(Eza + G.eidx(i, j + 1, 1));
-    const T ERL = ld(Eza + G.eidx(i + 1, j, 1)), ERR = ld(Eza + G.eidx(i + 1, j + 1, 1));
+    // each edge field is formed by its four cells: no pass and no array of its own
+    const T ELL = Ez2_at(a, i, j), ELR = Ez2_at(a, i, j + 1);
+    const T ERL = Ez2_at(a, i + 1, j), ERR = Ez2_at(a, i + 1, j + 1);
     T d2[2];
     cell_slopes2(a, IR, i, j, d2); const T drx = half * d2[0], dry = half * d2[1];
     cell_slopes2(a, IU, i, j, d2); const T dux = half * d2[0], duy = half * d2[1];
@@ -1102,9 +1101,10 @@ __global__ void __launch_bounds__(kThreads) k_trace2d(Geo G, const T *__restrict
 
     // scheme.f90:946-967
     const T sr0 = (-u * drx - dux * r) * dtdx + (-v * dry - dvy * r) * dtdy;
-    const T su0 = (-u * dux - dpx / r - B * dBx / r - C * dCx / r) * dtdx + (-v * duy + B * dAy / r) * dtdy;
-    const T sv0 = (-u * dvx + A * dBx / r) * dtdx + (-v * dvy - dpy / r - A * dAy / r - C * dCy / r) * dtdy;
-    const T sw0 = (-u * dwx + A * dCx / r) * dtdx + (-v * dwy + B * dCy / r) * dtdy;
+    const PerDensity<T, 10> d({dpx, B * dBx, C * dCx, B * dAy, A * dBx, dpy, A * dAy, C * dCy, A * dCx, B * dCy}, r);
+    const T su0 = (-u * dux - d(0, dpx) - d(1, B * dBx) - d(2, C * dCx)) * dtdx + (-v * duy + d(3, B * dAy)) * dtdy;
+    const T sv0 = (-u * dvx + d(4, A * dBx)) * dtdx + (-v * dvy - d(5, dpy) - d(6, A * dAy) - d(7, C * dCy)) * dtdy;
+    const T sw0 = (-u * dwx + d(8, A * dCx)) * dtdx + (-v * dwy + d(9, B * dCy)) * dtdy;
     const T sp0 = (-u * dpx - dux * gamma * p) * dtdx + (-v * dpy - dvy * gamma * p) * dtdy;
     const T sA0 = (u * dBy + B * duy - v * dAy - A * dvy) * dtdy;
     const T sB0 = (-u * dBx - B * dux + v * dAx + A * dvx) * dtdx;
@@ -1500,41 +1500,41 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 ? DG_RIEMANN_MINB64 
 // with an operand outside its range is done again by the *_ieee form (out of line: a kernel's
 // fast path carries only the call).  The kernels take Geo as a __grid_constant__, so that the
 // reference these calls pass needs no copy of it per thread.
-template <int kDir>
+template <int kDir, int kNd>
 __device__ __noinline__ void face_flux_ieee(const Geo &G, const double *core, long long cl, long long cr, int i,
                                             double dtd, double *out, long long fo) {
-    const CoreView<double> cv{core, kCore3};
+    const CoreView<double> cv{core, kNd == 3 ? kCore3 : kCore2};
     face_flux<double, true>(G, cv, cl, cr, kDir, i, dtd, out, fo);
 }
-template <int kDir>
+template <int kDir, int kNd = 3>
 __device__ __forceinline__ void face_flux_fast(const Geo &G, const double *core, long long cl, long long cr, int i,
                                                double dtd, double *__restrict__ out, long long fo) {
-    const CoreView<double> cv{core, kCore3};
+    const CoreView<double> cv{core, kNd == 3 ? kCore3 : kCore2};
     double ql[8], qr[8], f[8], pg;
     face_io(G, cv, cl, cr, kDir, ql, qr);
     FastMath m;
     hlld1d64(ql, qr, f, pg, G.gamma, G.ciso, G.iso, G.entho, m);
     if (m.bad()) {
-        face_flux_ieee<kDir>(G, core, cl, cr, i, dtd, out, fo);
+        face_flux_ieee<kDir, kNd>(G, core, cl, cr, i, dtd, out, fo);
         return;
     }
     flux_store(G, ql, qr, f, pg, kDir, i, dtd, out, fo);
 }
-template <int kDir>
+template <int kDir, int kNd>
 __device__ __noinline__ double edge_emf_ieee(const Geo &G, const double *core, long long cLL, long long cRL,
                                              long long cLR, long long cRR, int i, double dtd) {
-    const CoreView<double> cv{core, kCore3};
+    const CoreView<double> cv{core, kNd == 3 ? kCore3 : kCore2};
     return edge_emf<double, true>(G, cv, cLL, cRL, cLR, cRR, kDir, i, dtd);
 }
-template <int kDir>
+template <int kDir, int kNd = 3>
 __device__ __forceinline__ double edge_emf_fast(const Geo &G, const double *core, long long cLL, long long cRL,
                                                 long long cLR, long long cRR, int i, double dtd) {
-    const CoreView<double> cv{core, kCore3};
+    const CoreView<double> cv{core, kNd == 3 ? kCore3 : kCore2};
     Corners<double> c;
     edge_corners(G, cv, cLL, cRL, cLR, cRR, kDir, c);
     FastMath m;
     const double emf = hlld2d64(c, dtd, G.gamma, m);
-    if (m.bad()) return edge_emf_ieee<kDir>(G, core, cLL, cRL, cLR, cRR, i, dtd);
+    if (m.bad()) return edge_emf_ieee<kDir, kNd>(G, core, cLL, cRL, cLR, cRR, i, dtd);
     return edge_shear(G, c, emf, kDir, i, dtd);
 }
 
@@ -1680,20 +1680,40 @@ __global__ void __launch_bounds__(kThreads) k_riemann1d(Geo G, const T *__restri
     o[4] = f[6] * ds * dt; o[5] = pg; o[6] = f[3] * ds * dt; o[7] = f[5] * ds * dt; o[8] = f[7] * ds * dt;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kThreads) k_riemann2d(Geo G, const T *__restrict__ core, T *__restrict__ fx,
-                                                        T *__restrict__ fy, T *__restrict__ ez, const Scalars *S,
-                                                        int faces) {
+// 2D: the faces of x and y and the z edges as the rows of one grid (kind first + blockIdx.y; first = 2:
+// the edges alone).  2D grids are small: one thread that did its three solves in turn took 20 us on
+// 128 x 64 cells, 64 blocks of latency; the FP64 HLLD solves use round64.cuh as in 3D.
+template <typename T, bool kHLLD>
+__global__ void __launch_bounds__(kThreads) k_riemann2d(const __grid_constant__ Geo G, const T *__restrict__ core,
+                                                        T *__restrict__ fx, T *__restrict__ fy, T *__restrict__ ez,
+                                                        const Scalars *S, int first) {
     long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= G.fsz) return;
+    const int kind = first + blockIdx.y;
     const int j = (int)fdiv((unsigned)t, G.dFX) + 1;
     const int i = (int)((unsigned)t - (unsigned)(j - 1) * G.dFX.d) + 1;
+    if ((kind == 0 && j > G.ny) || (kind == 1 && i > G.nx)) return;
     const double dt = S->dt;
-    const CoreView<T> cv{core, kCore2};
-    const long long c = G.cidx(i, j, 1);
-    if (faces && j <= G.ny) face_flux(G, cv, G.cidx(i - 1, j, 1), c, 0, i, dt, fx, t);
-    if (faces && i <= G.nx) face_flux(G, cv, G.cidx(i, j - 1, 1), c, 1, i, dt, fy, t);
-    ez[t] = edge_emf(G, cv, G.cidx(i - 1, j - 1, 1), G.cidx(i, j - 1, 1), G.cidx(i - 1, j, 1), c, 2, i, dt);
+    const long long c = G.cidx(i, j, 1), l = c - 1, b = c - G.CX, lb = b - 1;
+    if constexpr (sizeof(T) == 8 && kHLLD) {
+        if (kind == 0) face_flux_fast<0, 2>(G, core, l, c, i, dt, fx, t);
+        else if (kind == 1) face_flux_fast<1, 2>(G, core, b, c, i, dt, fy, t);
+        else ez[t] = edge_emf_fast<2, 2>(G, core, lb, b, l, c, i, dt);
+    } else {
+        const CoreView<T> cv{core, kCore2};
+        if (kind == 0) face_flux<T, kHLLD>(G, cv, l, c, 0, i, dt, fx, t);
+        else if (kind == 1) face_flux<T, kHLLD>(G, cv, b, c, 1, i, dt, fy, t);
+        else ez[t] = edge_emf<T, kHLLD>(G, cv, lb, b, l, c, 2, i, dt);
+    }
+}
+template <typename T>
+void launch_riemann2d(const Geo &G, const T *core, T *fx, T *fy, T *ez, const Scalars *S, int faces, cudaStream_t s) {
+    const dim3 grid(nblocks(G.fsz, kThreads), faces ? 3 : 1);
+    const int first = faces ? 0 : 2;
+    if (G.iriemann == DG_RIEMANN_HLLD && G.iriemann2d == DG_RIEMANN_HLLD)
+        k_riemann2d<T, true><<<grid, kThreads, 0, s>>>(G, core, fx, fy, ez, S, first);
+    else
+        k_riemann2d<T, false><<<grid, kThreads, 0, s>>>(G, core, fx, fy, ez, S, first);
 }
 
 // ---------------------------------------------------------------------------
