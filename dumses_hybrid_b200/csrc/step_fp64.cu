@@ -43,28 +43,17 @@ __global__ void __launch_bounds__(kThreads) k_update3d(
     if (i <= nx && j <= ny && k <= nz) {
         // hydro update, scheme.f90:1783-1907
         const double Omega0 = G.omega0;
-        double lambda = 0.0, ratio = 0.0;
-        if (Omega0 > 0.0) {
-            lambda = Omega0 * dt; lambda = 2.5e-1 * lambda * lambda;
-            ratio = (one - lambda) / (one + lambda);
-        }
         const double dvloc = G.dvloc;  // one / (dx dy dz)
-        double ur = ld(U + c), uu = ld(U + sv * IU + c), uv = ld(U + sv * IV + c), uw = ld(U + sv * IW + c);
-        double up = ld(U + sv * IP + c);
-        if (Omega0 > 0.0) {
-            const double dsx = two * Omega0 * dt * uv / (one + lambda);
-            const double dsy = -(half * Omega0 * dt * uu) / (one + lambda);
-            uu = uu * ratio + dsx;
-            uv = uv * ratio + dsy;
-        }
-        const long long f0 = t;
+        double ur = ld(U + c), uw = ld(U + sv * IW + c), up = ld(U + sv * IP + c);
+        const double uu0 = ld(U + sv * IU + c), uv0 = ld(U + sv * IV + c);
         const long long fxr = (t + 1), fyr = (t + G.FX), fzr = (t + fxy);
         const double *FA[3] = {fx, fy, fz};
         const long long FR[3] = {fxr, fyr, fzr};
-        double pre[3];
+        double pre[3], dfn2[3], dfn3[3];  // the momentum increments of the three directions
+#pragma unroll
         for (int d = 0; d < 3; d++) {
             double L[6], R[6];
-            load6(FA[d] + f0 * kFluxRec3, L);
+            load6(FA[d] + t * kFluxRec3, L);
             load6(FA[d] + FR[d] * kFluxRec3, R);
             double rl = L[0], rr = R[0];
             if (d == 0 && shear) {
@@ -76,21 +65,49 @@ __global__ void __launch_bounds__(kThreads) k_update3d(
             ur = ur + (rl - rr) * dvloc;
             uw = uw + (L[4] * one - R[4] * one) * dvloc / one;
             up = up + (L[1] - R[1]) * dvloc;
-            if (Omega0 > 0.0) {
-                double dfn2 = (L[2] - R[2]) * dvloc;
-                if (d == 0) dfn2 = dfn2 + pre[0] * dvloc;
-                double dfn3 = (L[3] - R[3]) * dvloc;
-                if (d == 1) dfn3 = dfn3 + pre[1] * dvloc;
-                uu = uu + dfn2 / (one + lambda) + Omega0 * dt / (one + lambda) * dfn3;
-                uv = uv + dfn3 / (one + lambda) - 2.5e-1 * Omega0 * dt / (one + lambda) * dfn2;
-            } else {
-                uu = uu + (L[2] * one - R[2] * one) * dvloc / one;
-                uv = uv + (L[3] * one - R[3] * one) * dvloc / one;
-            }
+            dfn2[d] = (L[2] - R[2]) * dvloc;
+            dfn3[d] = (L[3] - R[3]) * dvloc;
         }
-        if (Omega0 == 0.0) {
-            uu = uu + pre[0] * dvloc;
-            uv = uv + pre[1] * dvloc;
+        double uu, uv;
+        if (Omega0 > 0.0) {
+            dfn2[0] = dfn2[0] + pre[0] * dvloc;
+            dfn3[1] = dfn3[1] + pre[1] * dvloc;
+            // the quotients by 1 + lambda share its reciprocal (round64.cuh)
+            auto rotate = [&](auto &m) {
+                double lambda = Omega0 * dt;
+                lambda = 2.5e-1 * lambda * lambda;
+                const double opl = one + lambda;
+                const auto io = m.rec(opl);
+                const double ratio = m.div(one - lambda, opl, io);
+                const double dsx = m.div(two * Omega0 * dt * uv0, opl, io);
+                const double dsy = m.div(-(half * Omega0 * dt * uu0), opl, io);
+                const double cu = m.div(Omega0 * dt, opl, io), cv = m.div(2.5e-1 * Omega0 * dt, opl, io);
+                uu = uu0 * ratio + dsx;
+                uv = uv0 * ratio + dsy;
+#pragma unroll
+                for (int d = 0; d < 3; d++) {
+                    uu = uu + m.div(dfn2[d], opl, io) + cu * dfn3[d];
+                    uv = uv + m.div(dfn3[d], opl, io) - cv * dfn2[d];
+                }
+            };
+            FastMath m;
+            rotate(m);
+            if (m.bad()) {
+                IeeeMath e;
+                rotate(e);
+            }
+        } else {
+            uu = uu0;
+            uv = uv0;
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                uu = uu + dfn2[d];
+                uv = uv + dfn3[d];
+            }
+            if (Omega0 == 0.0) {
+                uu = uu + pre[0] * dvloc;
+                uv = uv + pre[1] * dvloc;
+            }
         }
         uw = uw + pre[2] * dvloc;
         Un[c] = ur; Un[sv * IU + c] = uu; Un[sv * IV + c] = uv; Un[sv * IW + c] = uw; Un[sv * IP + c] = up;

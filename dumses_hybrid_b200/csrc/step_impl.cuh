@@ -265,14 +265,16 @@ __device__ __forceinline__ void finish_dt(const Geo &G, Scalars *S, unsigned lon
 
 // primitive variables of one cell in FP64 (scheme.f90:44-86); the right faces are the
 // neighbour's left faces (the frozen right z-face when ndim = 2)
-template <class Store>
-__device__ __forceinline__ void prim_cell(const Geo &G, const Store &U, long long c, double dt, double q[8]) {
-    const double one = 1.0, half = 0.5, two = 2.0;
+// (M: IeeeMath, or FastMath whose caller tests m.bad())
+template <class Store, class M>
+__device__ __forceinline__ void prim_cell(const Geo &G, const Store &U, long long c, double q[8], M &m) {
+    const double one = 1.0, half = 0.5, two = 2.0, dt = 0.0;
     const double d = U.getr(G, IR, c);
+    const auto id = m.rec(d);
     q[IR] = mx(d, kSmallr);
-    q[IU] = U.getr(G, IU, c) / d;
-    q[IV] = U.getr(G, IV, c) / d;
-    q[IW] = U.getr(G, IW, c) / d;
+    q[IU] = m.div(U.getr(G, IU, c), d, id);
+    q[IV] = m.div(U.getr(G, IV, c), d, id);
+    q[IW] = m.div(U.getr(G, IW, c), d, id);
     q[IA] = half * (U.getr(G, IA, c) + U.getr(G, IA, c + 1));
     // the right faces: the neighbour's left face, or the stored frozen copy (B_y, B_z in 1D,
     // B_z in 2D: the reference never refreshes those)
@@ -286,7 +288,7 @@ __device__ __forceinline__ void prim_cell(const Geo &G, const Store &U, long lon
         const double smallp = G.smallp;
         double eken = half * (q[IU] * q[IU] + q[IV] * q[IV] + q[IW] * q[IW]);
         double emag = half * (q[IA] * q[IA] + q[IB] * q[IB] + q[IC] * q[IC]);
-        double eint = (U.getr(G, IP, c) - emag) / d - eken;
+        double eint = m.div(U.getr(G, IP, c) - emag, d, id) - eken;
         q[IP] = mx((G.gamma - one) * q[IR] * eint, smallp);
     }
     if (G.omega0 > 0.0) {
@@ -297,15 +299,37 @@ __device__ __forceinline__ void prim_cell(const Geo &G, const Store &U, long lon
     }
 }
 
-// comp_speed, physics.f90:148-164
+// comp_speed, physics.f90:148-164; ir: the reciprocal of rho
+template <class M>
 __device__ __forceinline__ double comp_speed(double gamma, double rho, double p, double v, double bn, double bt1,
-                                             double bt2) {
+                                             double bt2, typename M::Rec ir, M &m) {
     const double half = 0.5;
-    double c2 = gamma * p / rho;
+    double c2 = m.div(gamma * p, rho, ir);
     double b2 = bn * bn + bt1 * bt1 + bt2 * bt2;
-    double d2 = half * (c2 + b2 / rho);
-    double cf = sqrt(d2 + sqrt(d2 * d2 - c2 * bn * bn / rho));
+    double d2 = half * (c2 + m.div(b2, rho, ir));
+    double cf = m.root(d2 + m.root(d2 * d2 - m.div(c2 * bn * bn, rho, ir)));
     return cf + fabs(v);
+}
+
+// the CFL time step of one cell from its primitive variables (physics.f90:42-121)
+template <class M>
+__device__ __forceinline__ double cell_dt(const Geo &G, const double q[8], M &m) {
+    const auto ir = m.rec(q[IR]);
+    // x / h, as a product where 1 / h is exact
+    auto per = [&](double x, double h, double rh, int p2) { return p2 ? x * rh : m.div(x, h, m.rec(h)); };
+    double velx = comp_speed(G.gamma, q[IR], q[IP], q[IU], q[IA], q[IB], q[IC], ir, m);
+    if (G.nx == 1) velx = 0.0;
+    if (G.ndim == 1) return m.div(G.dx, velx, m.rec(velx));  // physics.f90:101-103
+    double vely = comp_speed(G.gamma, q[IR], q[IP], q[IV], q[IB], q[IC], q[IA], ir, m);
+    if ((G.omega0 > 0.0) && !G.fargo) vely = vely + 1.5 * G.omega0 * (G.xmax - G.xmin) * 0.5;
+    if (G.ny == 1) vely = 0.0;
+    double sum = per(velx, G.dx, G.rdx, G.p2x) + per(vely, G.dy, G.rdy, G.p2y);
+    if (G.ndim == 3) {
+        double velz = comp_speed(G.gamma, q[IR], q[IP], q[IW], q[IC], q[IA], q[IB], ir, m);
+        if (G.nz == 1) velz = 0.0;
+        sum = sum + per(velz, G.dz, G.rdz, G.p2z);
+    }
+    return m.inv(sum);
 }
 
 // compute_dt (physics.f90:42-121) fused with the primitive variables of the next godunov
@@ -326,28 +350,21 @@ __global__ void __launch_bounds__(kThreads) k_prim_dt(Geo G, Store U, double *__
         j = (G.ndim > 1) ? j - 2 : 1;
         k = (G.ndim == 3) ? k - 2 : 1;
         const long long c = G.idx(i, j, k);
-        double q[8];
-        prim_cell(G, U, c, 0.0, q);
+        const bool active = i >= 1 && i <= G.nx && j >= 1 && j <= G.ny && k >= 1 && k <= G.nz;
+        double q[8], cdt = 1.0;
+        FastMath m;
+        prim_cell(G, U, c, q, m);
+        if (active) cdt = cell_dt(G, q, m);
+        if (m.bad()) {  // an operand outside the range of round64.cuh (or a bad state): the operators
+            IeeeMath e;
+            prim_cell(G, U, c, q, e);
+            if (active) cdt = cell_dt(G, q, e);
+        }
         if (chk(Q + c, 8) && chk(Q + G.sv * 7 + c, 8)) {
 #pragma unroll
             for (int v = 0; v < 8; v++) Q[G.sv * v + c] = q[v];
         }
-        if (i >= 1 && i <= G.nx && j >= 1 && j <= G.ny && k >= 1 && k <= G.nz) {
-            double velx = comp_speed(G.gamma, q[IR], q[IP], q[IU], q[IA], q[IB], q[IC]);
-            if (G.nx == 1) velx = 0.0;
-            double vely = comp_speed(G.gamma, q[IR], q[IP], q[IV], q[IB], q[IC], q[IA]);
-            if ((G.omega0 > 0.0) && !G.fargo) vely = vely + 1.5 * G.omega0 * (G.xmax - G.xmin) * 0.5;
-            if (G.ny == 1) vely = 0.0;
-            double cdt;
-            if (G.ndim == 1) {
-                cdt = G.dx / velx;  // physics.f90:101-103
-            } else if (G.ndim == 3) {
-                double velz = comp_speed(G.gamma, q[IR], q[IP], q[IW], q[IC], q[IA], q[IB]);
-                if (G.nz == 1) velz = 0.0;
-                cdt = 1.0 / (G.per_dx(velx) + G.per_dy(vely) + G.per_dz(velz));
-            } else {
-                cdt = 1.0 / (G.per_dx(velx) + G.per_dy(vely));
-            }
+        if (active) {
             if (!(cdt > 0.0)) bad = 1;  // NaN or non-positive
             else best = mn(best, cdt);
         }
@@ -385,7 +402,8 @@ __global__ void __launch_bounds__(kThreads) k_prim(Geo G, Store U, T *__restrict
     k = (G.ndim == 3) ? k - 2 : 1;
     const long long c = G.idx(i, j, k);
     double q[8];
-    prim_cell(G, U, c, 0.0, q);
+    IeeeMath m;
+    prim_cell(G, U, c, q, m);
 #pragma unroll
     for (int v = 0; v < 8; v++) Q[G.sv * v + c] = (T)q[v];
 }
