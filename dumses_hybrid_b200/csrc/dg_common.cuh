@@ -23,6 +23,13 @@ constexpr double kSmallc = 1.0e-10;  // commons.f90:49
 
 template <typename T> __host__ __device__ __forceinline__ T mn(T a, T b) { return a < b ? a : b; }
 template <typename T> __host__ __device__ __forceinline__ T mx(T a, T b) { return a > b ? a : b; }
+// x held at a floor; a NaN stays one.  FP32: one instruction instead of a compare and a select
+__device__ __forceinline__ double floored(double small, double x) { return mx(small, x); }
+__device__ __forceinline__ float floored(float small, float x) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(small), "f"(x));
+    return r;
+}
 __device__ __forceinline__ double sgn1(double x) { return copysign(1.0, x); }
 __device__ __forceinline__ float sgn1(float x) { return copysignf(1.0f, x); }
 __device__ __forceinline__ double fab(double x) { return fabs(x); }

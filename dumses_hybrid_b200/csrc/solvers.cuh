@@ -136,11 +136,10 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __
 __device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
 
 __device__ __forceinline__ void hlld1d_f(const float *ql, const float *qr, float *f, float &pg, float gamma,
-                                         float ciso, int iso) {
+                                         float ciso, int iso, float entho) {
     const float half = 0.5f, zero = 0.0f;
     const float2 r = p2(ql[0], qr[0]), u = p2(ql[2], qr[2]), v = p2(ql[4], qr[4]), b = p2(ql[5], qr[5]);
     const float2 w = p2(ql[6], qr[6]), c = p2(ql[7], qr[7]);
-    const float entho = 1.0f / (gamma - 1.0f);
     const float a = half * (ql[3] + qr[3]);
     const float aa = a * a;
     const float sgnm = copysignf(1.0f, a);
@@ -350,7 +349,7 @@ __device__ __forceinline__ void hlld1d64(const double *ql, const double *qr, dou
 template <typename T>
 __device__ void hlld1d(const T *ql, const T *qr, T *f, T &pg, T gamma, T ciso, int iso, T entho) {
     if constexpr (sizeof(T) == 4) {
-        hlld1d_f(ql, qr, f, pg, gamma, ciso, iso);
+        hlld1d_f(ql, qr, f, pg, gamma, ciso, iso, entho);
     } else {
         IeeeMath m;
         hlld1d64(ql, qr, f, pg, gamma, ciso, iso, entho, m);
@@ -367,6 +366,9 @@ struct Corners {
 
 template <typename T> __device__ __forceinline__ T mn4(T a, T b, T c, T d) { return mn(mn(mn(a, b), c), d); }
 template <typename T> __device__ __forceinline__ T mx4(T a, T b, T c, T d) { return mx(mx(mx(a, b), c), d); }
+// FP32: one instruction per minimum or maximum (a ternary is a compare and a select)
+__device__ __forceinline__ float mn4(float a, float b, float c, float d) { return fminf(fminf(fminf(a, b), c), d); }
+__device__ __forceinline__ float mx4(float a, float b, float c, float d) { return fmaxf(fmaxf(fmaxf(a, b), c), d); }
 
 template <typename T>
 __device__ T llf2d(const Corners<T> &c, T dt, T gamma, T ciso, int iso) {
@@ -397,23 +399,29 @@ __device__ T llf2d(const Corners<T> &c, T dt, T gamma, T ciso, int iso) {
     return emf * dt;
 }
 
-// FP32 form of hlld2d: per corner one reciprocal density shared by the x and y fast
-// speeds, reciprocal square roots of the star densities
+// FP32 form of hlld2d: per corner one reciprocal density, one sum of squares and one half trace
+// shared by the x and y fast speeds and the total pressure; reciprocal square roots of the star
+// densities.  Its kernel is bound by issue slots, so shared terms and one-instruction maxima count:
+// k_riemann3d at 256^3 2.02 -> 1.93 ms.
 __device__ __forceinline__ float hlld2d_f(const Corners<float> &c, float dt, float gamma) {
     const float half = 0.5f, zero = 0.0f, smallc = (float)kSmallc;
-    const float iLL = 1.0f / c.rLL, iLR = 1.0f / c.rLR, iRL = 1.0f / c.rRL, iRR = 1.0f / c.rRR;
-    const float cfx = sqrtf(mx4(cfast2_r(gamma, c.pLL, iLL, c.ALL, c.BLL, c.CLL), cfast2_r(gamma, c.pLR, iLR, c.ALR, c.BLR, c.CLR),
-                                cfast2_r(gamma, c.pRL, iRL, c.ARL, c.BRL, c.CRL), cfast2_r(gamma, c.pRR, iRR, c.ARR, c.BRR, c.CRR)));
-    const float cfy = sqrtf(mx4(cfast2_r(gamma, c.pLL, iLL, c.BLL, c.ALL, c.CLL), cfast2_r(gamma, c.pLR, iLR, c.BLR, c.ALR, c.CLR),
-                                cfast2_r(gamma, c.pRL, iRL, c.BRL, c.ARL, c.CRL), cfast2_r(gamma, c.pRR, iRR, c.BRR, c.ARR, c.CRR)));
+    auto corner = [&](float r, float p, float a, float b, float cc, float &fx, float &fy, float &pt) {
+        const float ir = 1.0f / r, a2 = a * a, b2 = b * b, s2 = a2 + b2 + cc * cc;
+        const float c2 = gamma * p * ir, d2 = half * (c2 + s2 * ir), dd = d2 * d2, k = c2 * ir;
+        fx = d2 + sqrtf(fmaxf(dd - k * a2, zero));
+        fy = d2 + sqrtf(fmaxf(dd - k * b2, zero));
+        pt = p + half * s2;
+    };
+    float xLL, xLR, xRL, xRR, yLL, yLR, yRL, yRR, PtotLL, PtotLR, PtotRL, PtotRR;
+    corner(c.rLL, c.pLL, c.ALL, c.BLL, c.CLL, xLL, yLL, PtotLL);
+    corner(c.rLR, c.pLR, c.ALR, c.BLR, c.CLR, xLR, yLR, PtotLR);
+    corner(c.rRL, c.pRL, c.ARL, c.BRL, c.CRL, xRL, yRL, PtotRL);
+    corner(c.rRR, c.pRR, c.ARR, c.BRR, c.CRR, xRR, yRR, PtotRR);
+    const float cfx = sqrtf(mx4(xLL, xLR, xRL, xRR)), cfy = sqrtf(mx4(yLL, yLR, yRL, yRR));
     const float SL = mn4(c.uLL, c.uLR, c.uRL, c.uRR) - cfx;
     const float SR = mx4(c.uLL, c.uLR, c.uRL, c.uRR) + cfx;
     const float SB = mn4(c.vLL, c.vLR, c.vRL, c.vRR) - cfy;
     const float ST = mx4(c.vLL, c.vLR, c.vRL, c.vRR) + cfy;
-    const float PtotLL = c.pLL + half * (c.ALL * c.ALL + c.BLL * c.BLL + c.CLL * c.CLL);
-    const float PtotLR = c.pLR + half * (c.ALR * c.ALR + c.BLR * c.BLR + c.CLR * c.CLR);
-    const float PtotRL = c.pRL + half * (c.ARL * c.ARL + c.BRL * c.BRL + c.CRL * c.CRL);
-    const float PtotRR = c.pRR + half * (c.ARR * c.ARR + c.BRR * c.BRR + c.CRR * c.CRR);
     const float rcLLx = c.rLL * (c.uLL - SL), rcRLx = c.rRL * (SR - c.uRL);
     const float rcLRx = c.rLR * (c.uLR - SL), rcRRx = c.rRR * (SR - c.uRR);
     const float rcLLy = c.rLL * (c.vLL - SB), rcLRy = c.rLR * (ST - c.vLR);

@@ -323,10 +323,8 @@ __device__ __forceinline__ float hl_diff(HL a, HL b) { return (a.h - b.h) + (a.l
 // uin_slope (fargo.f90:266-280) from the (hi, lo) values at j-1, j, j+1, on differences
 __device__ __forceinline__ float slope_hl(int ist, HL m, HL c, HL p) {
     if (ist == 0) return 0.0f;
-    const float sl = (float)ist;
-    const float dlft = sl * hl_diff(c, m), drgt = sl * hl_diff(p, c);
-    const float dcen = 0.5f * (dlft + drgt) / sl;
-    const float dlim = (dlft * drgt <= 0.0f) ? 0.0f : fminf(fabsf(dlft), fabsf(drgt));
+    const float dl = hl_diff(c, m), dr = hl_diff(p, c), dcen = 0.5f * (dl + dr);
+    const float dlim = dl * dr <= 0.0f ? 0.0f : (float)ist * fminf(fabsf(dl), fabsf(dr));
     return copysignf(fminf(dlim, fabsf(dcen)), dcen);
 }
 // emfx (i in 1..nx, k in 1..nz+1) and emfz (i in 1..nx+1, k in 1..nz) over j in 1..ny+1,
