@@ -50,6 +50,7 @@ static_assert(kNHid >= 1 && kNHid <= 3, "one to three hidden layers");
 
 struct FaceUnits {
     float rho0, a0, b0, jump;  // interface units and the jump size J
+    float irl, irr;            // 1 / rho of the two states
 };
 
 constexpr float kTinyJump = 1e-20f;
@@ -75,7 +76,9 @@ __device__ __forceinline__ FaceUnits face_inputs(const float *ql, const float *q
     const float b2r = bn * bn + qr[5] * qr[5] + qr[7] * qr[7];
     FaceUnits u;
     u.rho0 = 0.5f * (ql[0] + qr[0]);
-    u.a0 = sqrtf(fmaxf((gamma * pl + b2l) / ql[0], (gamma * pr + b2r) / qr[0]));
+    u.irl = 1.0f / ql[0];
+    u.irr = 1.0f / qr[0];
+    u.a0 = sqrtf(fmaxf((gamma * pl + b2l) * u.irl, (gamma * pr + b2r) * u.irr));
     u.b0 = sqrtf(u.rho0) * u.a0;
     const float ir = 1.0f / u.rho0, ia = 1.0f / u.a0, ip = ir * ia * ia, ib = 1.0f / u.b0;
     // scaled left and right: rho, u_n, v_t1, v_t2, P, B_t1, B_t2
@@ -121,6 +124,40 @@ __device__ __forceinline__ void base_fluxes(const T *ql, const T *qr, T gamma, T
     dis[7] = T(0);
 }
 
+// the same for the face kernel (FP32): one reciprocal per density (face_inputs'), entho = 1 / (gamma - 1)
+// formed once, and only the terms the outputs need
+__device__ __forceinline__ void base_fluxes_f(const float *ql, const float *qr, float gamma, float ciso, int iso,
+                                              float entho, const FaceUnits &un, float b[kOut], float dis[kOut]) {
+    const float a = ql[3], aa = a * a;
+    float fl[7], cl[7], fr[7], cr[7], pt[2];
+    auto side = [&](const float *q, float ir, float *f, float *c, float &ptot) {
+        const float r = q[0], u = q[2], v = q[4], w = q[6], bt = q[5], ct = q[7];
+        const float p = iso ? r * (ciso * ciso) : q[1];
+        const float b2 = aa + bt * bt + ct * ct, emag = 0.5f * b2;
+        c[0] = r; c[2] = r * u; c[3] = r * v; c[4] = bt; c[5] = r * w; c[6] = ct;
+        c[1] = p * entho + 0.5f * (c[2] * u + c[3] * v + c[5] * w) + emag;
+        ptot = p + emag;
+        f[0] = c[2];
+        f[1] = (c[1] + ptot) * u - a * (u * a + v * bt + w * ct);
+        f[2] = c[2] * u + ptot - aa;
+        f[3] = c[2] * v - a * bt;
+        f[4] = bt * u - a * v;
+        f[5] = c[2] * w - a * ct;
+        f[6] = ct * u - a * w;
+        const float c2 = gamma * p * ir, d2 = 0.5f * (c2 + b2 * ir);
+        return sqrtf(d2 + sqrtf(fmaxf(d2 * d2 - c2 * aa * ir, 0.0f))) + fabsf(u);
+    };
+    const float vl = side(ql, un.irl, fl, cl, pt[0]), vr = side(qr, un.irr, fr, cr, pt[1]);
+    const float hv = 0.5f * fmaxf(vl, vr);
+#pragma unroll
+    for (int n = 0; n < 7; n++) {
+        dis[n] = hv * (cr[n] - cl[n]);
+        b[n] = 0.5f * (fl[n] + fr[n]) - dis[n];
+    }
+    b[7] = 0.5f * (pt[0] + pt[1]);
+    dis[7] = 0.0f;
+}
+
 // dissipation gate: per flux component, the learned correction k (in units of scale x J)
 // must move the flux from LLF towards the central flux, no further than the whole LLF
 // dissipation dn (same units), up to eps = 5% of the largest |dn|.  A flux outside that
@@ -155,23 +192,6 @@ struct Gates {
     float compress;              // u_nR - u_nL below -compress * a0 marks a shock: HLLD
     float margin;                // envelope margin (fraction of its width)
 };
-
-// true when the interface is smooth and inside the network's training envelope
-__device__ __forceinline__ bool gate_inputs(const Gates &g, const float *ql, const float *qr, float ciso, int iso,
-                                            const FaceUnits &u, const float x[kIn]) {
-    const float rl = ql[0], rr = qr[0];
-    const float pl = iso ? rl * (ciso * ciso) : ql[1], pr = iso ? rr * (ciso * ciso) : qr[1];
-    if (!(rl > 0.0f && rr > 0.0f && pl > 0.0f && pr > 0.0f)) return false;           // positivity
-    if (fabsf(pl - pr) > g.jump * fminf(pl, pr)) return false;                         // pressure jump
-    if (fabsf(rl - rr) > g.jump * fminf(rl, rr)) return false;                         // density jump
-    if (qr[2] - ql[2] < -g.compress * u.a0) return false;                              // compression
-#pragma unroll
-    for (int n = 0; n < kIn; n++) {
-        const float w = g.margin * (g.xmax[n] - g.xmin[n]);
-        if (!(x[n] >= g.xmin[n] - w && x[n] <= g.xmax[n] + w)) return false;          // confidence: envelope
-    }
-    return true;
-}
 
 // SmeLU, the smooth ReLU of Shamir, Lin, Coviello and Chen ("Smooth activations and
 // reproducibility in deep networks", 2020) with half-width 1:
@@ -219,8 +239,25 @@ struct NetView {
     const __nv_bfloat16 *bt[kNHid]; // hidden-layer bias operands, blocked K-major [kHid][kBiasK]
     const float *b[kNL];            // biases
     Gates gates;
+    float xlo[kIn], xhi[kIn];       // the input envelope with its margin
     Scaling sc;
 };
+
+// true when the interface is smooth and inside the network's training envelope
+__device__ __forceinline__ bool gate_inputs(const NetView &nv, const float *ql, const float *qr, float ciso, int iso,
+                                            const FaceUnits &u, const float x[kIn]) {
+    const Gates &g = nv.gates;
+    const float rl = ql[0], rr = qr[0];
+    const float pl = iso ? rl * (ciso * ciso) : ql[1], pr = iso ? rr * (ciso * ciso) : qr[1];
+    if (!(rl > 0.0f && rr > 0.0f && pl > 0.0f && pr > 0.0f)) return false;           // positivity
+    if (fabsf(pl - pr) > g.jump * fminf(pl, pr)) return false;                         // pressure jump
+    if (fabsf(rl - rr) > g.jump * fminf(rl, rr)) return false;                         // density jump
+    if (qr[2] - ql[2] < -g.compress * u.a0) return false;                              // compression
+#pragma unroll
+    for (int n = 0; n < kIn; n++)
+        if (!(x[n] >= nv.xlo[n] && x[n] <= nv.xhi[n])) return false;                   // confidence: envelope
+    return true;
+}
 
 }  // namespace nn
 }  // namespace dg

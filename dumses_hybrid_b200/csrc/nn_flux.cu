@@ -1352,6 +1352,11 @@ int dg_nn_view(const dg_nn *n, dg::nn::NetView *v) {
     for (int l = 0; l < kNL; l++) { v->wt[l] = n->Wt[l]; v->b[l] = n->b[l]; }
     for (int l = 0; l < kNHid; l++) v->bt[l] = n->Bt[l];
     v->gates = n->gates;
+    for (int q = 0; q < kIn; q++) {
+        const float w = n->gates.margin * (n->gates.xmax[q] - n->gates.xmin[q]);
+        v->xlo[q] = n->gates.xmin[q] - w;
+        v->xhi[q] = n->gates.xmax[q] + w;
+    }
     v->sc = n->sc;
     return DG_OK;
 }

@@ -639,7 +639,7 @@ __global__ void __launch_bounds__(128 * kNWG, 1) k_nn_faces(Geo G, const float *
     }
     __syncthreads();
     const CoreView<float> cv{core, G.ndim == 3 ? kCore3 : kCore2};
-    const float gamma = (float)G.gamma, ciso = (float)G.ciso;
+    const float gamma = (float)G.gamma, ciso = (float)G.ciso, entho = (float)G.entho;
     const double dt = S->dt;
     unsigned ph = 0;
     unsigned long long nface = 0, nfall = 0;
@@ -660,7 +660,7 @@ __global__ void __launch_bounds__(128 * kNWG, 1) k_nn_faces(Geo G, const float *
                   : (d == 1) ? (i <= G.nx && (G.ndim == 2 || k <= G.nz)) : (i <= G.nx && j <= G.ny);
         }
         float ql[8], qr[8], x[nn::kInPad], base[nn::kOut], dis[nn::kOut];
-        nn::FaceUnits u{1.0f, 1.0f, 1.0f, 0.0f};
+        nn::FaceUnits u{1.0f, 1.0f, 1.0f, 0.0f, 1.0f, 1.0f};
         bool use = false;
 #pragma unroll
         for (int n = 0; n < nn::kInPad; n++) x[n] = 0.0f;
@@ -682,8 +682,8 @@ __global__ void __launch_bounds__(128 * kNWG, 1) k_nn_faces(Geo G, const float *
                 face_io(G, cv, cl, cr, d, ql, qr);
             }
             u = nn::face_inputs(ql, qr, gamma, ciso, G.iso, x);
-            use = nn::gate_inputs(nv.gates, ql, qr, ciso, G.iso, u, x);
-            nn::base_fluxes<float>(ql, qr, gamma, ciso, G.iso, base, dis);
+            use = nn::gate_inputs(nv, ql, qr, ciso, G.iso, u, x);
+            nn::base_fluxes_f(ql, qr, gamma, ciso, G.iso, entho, u, base, dis);
         }
         if constexpr (kNStage) {  // the next tile's values, in flight while this tile's layers run
             stage_face(G, core, cv.nf, d, (tile + tstride) * 128 + wt, stg);
@@ -755,12 +755,17 @@ __global__ void __launch_bounds__(128 * kNWG, 1) k_nn_faces(Geo G, const float *
         if (valid) {
             bool acc = use;
             float F[nn::kOut], dn[nn::kOut];
+            // scale x J and its reciprocal: four different ones (momenta and p*_T share theirs)
+            const float m = u.rho0 * u.a0, sj4[4] = {m * u.jump, m * u.a0 * u.a0 * u.jump, m * u.a0 * u.jump, u.b0 * u.a0 * u.jump};
+            float ij4[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) ij4[q] = sj4[q] > 0.0f ? 1.0f / sj4[q] : 0.0f;
 #pragma unroll
             for (int c = 0; c < nn::kOut; c++) {
+                constexpr int kind[nn::kOut] = {0, 1, 2, 2, 3, 2, 3, 2};
                 acc = acc && fabsf(y[c]) <= 1.5f * nv.gates.ymax;  // confidence: inside the training range
-                const float sj = nn::out_scale(u, c) * u.jump;
-                F[c] = base[c] + sj * y[c];
-                dn[c] = (sj > 0.0f) ? dis[c] / sj : 0.0f;
+                F[c] = base[c] + sj4[kind[c]] * y[c];
+                dn[c] = dis[c] * ij4[kind[c]];
                 acc = acc && isfinite(F[c]);
             }
             acc = acc && F[7] > 0.0f;                      // positive star pressure
