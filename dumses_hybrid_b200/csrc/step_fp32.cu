@@ -11,6 +11,7 @@
 #include "step_impl.cuh"
 #include "nn_features.cuh"
 #include "nn_umma.cuh"
+#include "riemann32.cuh"
 
 namespace dg {
 namespace f32 {
@@ -895,6 +896,9 @@ int launch_godunov(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
             }
             if (hlld) TIMED(KS_RIEMANN, s, (k_edges3d<float, true><<<nb, kThreads, 0, s>>>(G, core, ex, ey, ez, B.S)));
             else TIMED(KS_RIEMANN, s, (k_edges3d<float, false><<<nb, kThreads, 0, s>>>(G, core, ex, ey, ez, B.S)));
+        } else if (hlld && riemann_pairs(G)) {
+            const unsigned np = nblocks((G.csz - (long long)G.CX * G.CY) / 2, kThreads);
+            TIMED(KS_RIEMANN, s, (k_riemann32<<<np, kThreads, 0, s>>>(G, core, fx, fy, fz, ex, ey, ez, B.S, faces)));
         } else if (hlld) {
             TIMED(KS_RIEMANN, s, (k_riemann3d<float, true><<<nb, kThreads, 0, s>>>(G, core, fx, fy, fz, ex, ey, ez, B.S, faces)));
         } else {
@@ -907,7 +911,10 @@ int launch_godunov(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
         for (int d = 0; d < G.ndim; d++) {
             // the list's length is on the device: a grid-stride grid of 16 blocks per SM, above the ~7
             // that stay resident, so that every SM has its full share of the scattered gathers in flight
-            TIMED(KS_NN_FALLBACK, s, (k_nn_fallback<<<148 * 16, kThreads, 0, s>>>(G, core, fl[d], B.fb_list[d], B.nn_count, d, B.S)));
+            if (G.ndim == 2 || !riemann_pairs(G)) TIMED(KS_NN_FALLBACK, s, (k_nn_fallback<<<148 * 16, kThreads, 0, s>>>(G, core, fl[d], B.fb_list[d], B.nn_count, d, B.S)));
+            else if (d == 0) TIMED(KS_NN_FALLBACK, s, (k_nn_fallback32<0><<<148 * 16, kThreads, 0, s>>>(G, core, fl[d], B.fb_list[d], B.nn_count, B.S)));
+            else if (d == 1) TIMED(KS_NN_FALLBACK, s, (k_nn_fallback32<1><<<148 * 16, kThreads, 0, s>>>(G, core, fl[d], B.fb_list[d], B.nn_count, B.S)));
+            else TIMED(KS_NN_FALLBACK, s, (k_nn_fallback32<2><<<148 * 16, kThreads, 0, s>>>(G, core, fl[d], B.fb_list[d], B.nn_count, B.S)));
             n++;
         }
     }
