@@ -92,3 +92,24 @@ def test_solves_outside_the_straight_line_range(name, iso):
         ug = g.download()
     assert tg == t
     compare_states(ug, o.uin, p)
+
+
+@pytest.mark.parametrize("iso", [False, True])
+@pytest.mark.parametrize("name", ["units_large", "tiny_field", "mixed_cells", "near_unity"])
+def test_2d_solves_outside_the_straight_line_range(name, iso):
+    kw = dict(iso=1, ciso=2.0**60 if name == "units_large" else 1.0) if iso else {}
+    p = Params(ndim=2, nx=33, ny=18, nz=1, xmin=0, xmax=1, ymin=0, ymax=1, courant=0.4, **kw)
+    u0 = np.asfortranarray(variant(name, condinit(p, "field_loop")))
+    o = Oracle(p)
+    o.set_state(u0)
+    o.boundary(0.0, 0.0)
+    t = 0.0
+    for _ in range(2):
+        t, _ = o.step(t)
+    with Context(p) as g:
+        g.upload(u0)
+        g.boundary(0.0, 0.0)
+        tg, _ = g.run(2, 0.0)
+        ug = g.download()
+    assert tg == t
+    compare_states(ug, o.uin, p)
