@@ -969,7 +969,7 @@ int launch_fargo(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
 }
 
 int launch_boundary(const Geo &G, const Bufs &B, int cur, cudaStream_t s, int advance) {
-    TIMED(KS_BOUNDARY, s, (k_boundary<StoreHL><<<nblocks(ghost_cells(G), kThreads), kThreads, 0, s>>>(G, st(B, cur), B.nv, B.S, advance)));
+    TIMED(KS_BOUNDARY, s, run_boundary(G, st(B, cur), B.nv, B.S, advance, s));
     return 1;
 }
 

@@ -1800,12 +1800,18 @@ __host__ __device__ __forceinline__ long long ghost_cells(const Geo &G) {
     return nA + nB + nC;
 }
 
+// Variables a thread fills (kVars; blockIdx.y: which).  Copies: all of them, one round of loads in flight.
+// The shear remap reads four rows of each and is bound by the latency of those loads: four variables a
+// thread double the warps (and take 56 registers instead of 80 in FP32) for repeated index arithmetic.  FP32 shearing box
+// 128^3 45.8 -> 35.2 us, 256^3 127 -> 111, FP64 128^3 27.0 -> 25.3; two variables 37.3, 120 and 31.1, one
+// 41.4, 128 and 36.1.  With copies alone four are slower (FP64 64^3 9.9 against 8.9 us).
 constexpr int kMaxVars = 10;  // stored state variables: 8, plus the frozen right-face B (z in 2D, y and z in 1D)
-template <class Store>
+constexpr int kShearVars = 4;
+template <class Store, int kVars>
 __global__ void __launch_bounds__(kThreads) k_boundary(Geo G, Store U, int nv, Scalars *S, int advance) {
     long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= ghost_cells(G)) return;
-    if (advance && t == 0) S->time = S->time + S->dt;  // the last kernel of a step; no thread here reads time
+    if (advance && t == 0 && blockIdx.y == 0) S->time = S->time + S->dt;  // the last kernel of a step; no thread here reads time
     // the ghost counts of any grid that fits a GPU are far below 2^32: 32-bit index arithmetic
     const unsigned NX = G.NX, NY = G.NY;
     const unsigned nA = (G.ndim == 3) ? 6u * NX * NY : 0u;
@@ -1839,15 +1845,16 @@ __global__ void __launch_bounds__(kThreads) k_boundary(Geo G, Store U, int nv, S
     const long long c = G.idx(i, j, k);
     // every value is read (from active cells, or the outer x face that no thread writes)
     // before the first store, so the loads of all variables are in flight together
-    double out[kMaxVars];
-    if (!gx || G.bc[0] != DG_BC_SHEARINGBOX) {
+    double out[kVars];
+    const int v0 = kVars == kMaxVars ? 0 : blockIdx.y * kVars;
+    if (kVars == kMaxVars || !gx || G.bc[0] != DG_BC_SHEARINGBOX) {  // run_boundary: all at once is for copies
         const long long src = G.idx(map_bc(G.bc[0], i, G.nx), jj, kk);
 #pragma unroll
-        for (int v = 0; v < kMaxVars; v++)
-            if (v < nv) out[v] = U.get(G, v, src);
+        for (int n = 0; n < kVars; n++)
+            if (v0 + n < nv) out[n] = U.get(G, v0 + n, src);
 #pragma unroll
-        for (int v = 0; v < kMaxVars; v++)
-            if (v < nv) U.set(G, v, c, out[v]);
+        for (int n = 0; n < kVars; n++)
+            if (v0 + n < nv) U.set(G, v0 + n, c, out[n]);
         return;
     }
     // shear-periodic x ghost (only with ndim = 3; shearingbox.f90:62-147): the remapped rows,
@@ -1875,32 +1882,43 @@ __global__ void __launch_bounds__(kThreads) k_boundary(Geo G, Store U, int nv, S
     const double lambda = half * eps * (eps - one);
     const int st = mn(G.slope_type, 2);
     auto row = [&](int r) { return G.idx(src, map_bc(G.bc[1], r, ny), kk); };
-    // rows of the two values and of shearing_slope at each (shearingbox.f90:415-430, 493-499)
-    const long long cm = row(jr - 1), c0 = row(jr), cp = row(jr + 1);
-    const long long dm = row(jrp - 1), d0 = row(jrp), dp = row(jrp + 1);
+    // the rows of the two values, neighbours in y whichever of them wrapped, and the rows beyond either
+    // that shearing_slope takes (shearingbox.f90:415-430, 493-499)
+    const long long rm = row(jr - 1), ra = row(jr), rb = row(jrp), rp = row(jrp + 1);
     // the outer face keeps its own (CT-updated) value; ghost j/k copy it
     const bool outer = (i == nx + 1);
     const bool keep_a = outer && jj == j && kk == k;
     const long long ca = G.idx(i, jj, kk);
 #pragma unroll
-    for (int v = 0; v < kMaxVars; v++) {
+    for (int n = 0; n < kVars; n++) {
+        const int v = v0 + n;
         if (v >= nv) continue;
         if (v == IA && outer) {
-            out[v] = U.get(G, v, ca);
-        } else if (v == IB) {  // By: one-sided slope
-            const double a0 = U.get(G, v, c0), a1 = U.get(G, v, cp);
-            out[v] = a0 + eps * (st == 0 ? 0.0 : a1 - a0);
+            out[n] = U.get(G, v, ca);
+            continue;
+        }
+        const double a = U.get(G, v, ra), b = U.get(G, v, rb);
+        if (v == IB) {  // By: one-sided slope
+            out[n] = a + eps * (st == 0 ? 0.0 : b - a);
         } else {
-            const double am = U.get(G, v, cm), a0 = U.get(G, v, c0), ap = U.get(G, v, cp);
-            const double bm = U.get(G, v, dm), b0 = U.get(G, v, d0), bp = U.get(G, v, dp);
-            const double sa = st == 0 ? 0.0 : limit1<double>((double)st, am, a0, ap);
-            const double sb = st == 0 ? 0.0 : limit1<double>((double)st, bm, b0, bp);
-            out[v] = (one - eps) * a0 + eps * b0 + lambda * (lower ? sa - sb : sb - sa);
+            const double m = U.get(G, v, rm), p = U.get(G, v, rp);
+            const double sa = st == 0 ? 0.0 : limit1<double>((double)st, m, a, b);
+            const double sb = st == 0 ? 0.0 : limit1<double>((double)st, a, b, p);
+            out[n] = (one - eps) * a + eps * b + lambda * (lower ? sa - sb : sb - sa);
         }
     }
 #pragma unroll
-    for (int v = 0; v < kMaxVars; v++)
-        if (v < nv && !(v == IA && keep_a)) U.set(G, v, c, out[v]);
+    for (int n = 0; n < kVars; n++)
+        if (v0 + n < nv && !(v0 + n == IA && keep_a)) U.set(G, v0 + n, c, out[n]);
+}
+
+template <class Store>
+void run_boundary(const Geo &G, Store U, int nv, Scalars *S, int advance, cudaStream_t s) {
+    const unsigned nb = nblocks(ghost_cells(G), kThreads);
+    if (G.bc[0] == DG_BC_SHEARINGBOX)
+        k_boundary<Store, kShearVars><<<dim3(nb, (nv + kShearVars - 1) / kShearVars), kThreads, 0, s>>>(G, U, nv, S, advance);
+    else
+        k_boundary<Store, kMaxVars><<<nb, kThreads, 0, s>>>(G, U, nv, S, advance);
 }
 
 // right-face B (uin vars 9-11) of the reference layout, from the stored left faces
