@@ -845,12 +845,6 @@ int launch_dt(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
     return 1;
 }
 
-// 3D Riemann work as two kernels (faces, then edges) instead of one
-#ifndef DG_RIEMANN_SPLIT32
-#define DG_RIEMANN_SPLIT32 0
-#endif
-constexpr bool kRiemannSplit32 = DG_RIEMANN_SPLIT32 != 0;
-
 int launch_godunov(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
     const StoreHL U = st(B, cur), Un = st(B, cur ^ 1);
     float *Q = (float *)B.Q, *core = (float *)B.core;
@@ -888,15 +882,7 @@ int launch_godunov(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
         // HLLD/HLLD (the reference's default and every benchmark) runs kernels without the other solvers
         const bool hlld = G.iriemann == DG_RIEMANN_HLLD && G.iriemann2d == DG_RIEMANN_HLLD;
         const unsigned nb = nblocks(G.fsz, kThreads);
-        if (kRiemannSplit32) {
-            if (faces) {
-                if (hlld) TIMED(KS_RIEMANN, s, (k_faces3d<float, true><<<nb, kThreads, 0, s>>>(G, core, fx, fy, fz, B.S)));
-                else TIMED(KS_RIEMANN, s, (k_faces3d<float, false><<<nb, kThreads, 0, s>>>(G, core, fx, fy, fz, B.S)));
-                n++;
-            }
-            if (hlld) TIMED(KS_RIEMANN, s, (k_edges3d<float, true><<<nb, kThreads, 0, s>>>(G, core, ex, ey, ez, B.S)));
-            else TIMED(KS_RIEMANN, s, (k_edges3d<float, false><<<nb, kThreads, 0, s>>>(G, core, ex, ey, ez, B.S)));
-        } else if (hlld && riemann_pairs(G)) {
+        if (hlld && riemann_pairs(G)) {
             const unsigned np = nblocks((G.csz - (long long)G.CX * G.CY) / 2, kThreads);
             TIMED(KS_RIEMANN, s, (k_riemann32<<<np, kThreads, 0, s>>>(G, core, fx, fy, fz, ex, ey, ez, B.S, faces)));
         } else if (hlld) {

@@ -275,8 +275,9 @@ __global__ void __launch_bounds__(kThreads) k_update2d(Geo G, const double *__re
 // mostly share one kind's code (a sixth of the whole) while the chunk's trace core, read from HBM by
 // the first kind, is in L2 for the others: 0.88 GB of HBM reads at 128^3 against 2.0 GB for a kernel
 // per kind.  At 256^3 (MRI, FARGO): six kernels with IEEE operators 7.21 ms, with round64.cuh 5.96,
-// this grid 5.69 (chunks of 148 tiles 6.65, 370 5.83, 1480 5.75, 2960 5.79; 4 blocks per SM instead
-// of 5: 5.87; 6 blocks, as six kernels: 7.20 with spills); at 64^3 0.184 -> 0.110 ms, where a kernel
+// this grid 5.69 (5.9 since round64.cuh rounds its reciprocals correctly; before that chunks of 148
+// tiles 6.65, 370 5.83, 1480 5.75, 2960 5.79; 4 blocks per SM instead of 5: 5.87; 6 blocks, as six
+// kernels: 7.20 with spills); at 64^3 0.184 -> 0.110 ms, where a kernel
 // per kind is less than one wave.
 #ifndef DG_RIEMANN_CHUNK64
 #define DG_RIEMANN_CHUNK64 740
