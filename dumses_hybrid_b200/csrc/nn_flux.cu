@@ -289,12 +289,19 @@ __global__ void __launch_bounds__(128) k_loss(const float *__restrict__ Y, const
 // activation derivatives to each other through HBM and spent their time in the epilogues' 2-byte and
 // strided stores and per-column shuffle sums: 156 us for a batch of 65536 (17-64-64-8), where the
 // products themselves are a few microseconds of tensor time (batch of 65536: an Adam step 206 us then,
-// 48 us now, 40 of them in this kernel).  Here a persistent block takes
+// 52 us now, 41 of them in this kernel).  Here a persistent block takes
 // 128-row tiles through the whole pass: the activations stay in shared memory as the operands of the
 // next product, the pre-activations stay in tensor memory for the backward pass, and the weight
-// gradients accumulate in tensor memory over the block's tiles.  Only the sampled rows are read and
-// one gradient per block is written.  Bound by the latency of its chain of products and epilogues:
-// four warpgroups share a tile, each with 16 of its columns, and the next tile's rows are in flight.
+// gradients accumulate in tensor memory over a split of the batch.  Only the sampled rows are read and
+// one weight gradient per split and the bias and loss sums of each tile are written.  Bound by the
+// latency of its chain of products and epilogues: four warpgroups share a tile, each with 16 of its
+// columns, and the next tile's rows are in flight.
+//
+// The order of the FP32 sums is the kernel chain's, so that a training run gives the same numbers by
+// either: through the rounding of the weights to BF16 another grouping (every 148th tile in a block)
+// moved the loss of 40 steps by 2.9e-5.  A split is split_rows() consecutive rows, one accumulation in the tensor core;
+// k_adam adds the splits in order; bias and loss sums are per tile (32 rows by a fixed tree, then the
+// four warps in order) and added in tile order.
 //
 // Shared-memory operands are blocked K-major as in nn_umma.cuh.  The transposed operands (reduction
 // over the tile's 128 rows) hold kHid rows; as the A operand of an M = 128 product their rows kHid..127
@@ -307,7 +314,8 @@ constexpr int train_weights() {  // bytes of the forward and backward weight ope
     for (int l = 0; l < kNL; l++) b += layer_k(l) * layer_n(l) * 2 * (l > 0 ? 2 : 1);
     return b;
 }
-constexpr int kTrainSmem = 2 * kTrainX + (2 + kNHid) * kTrainH + 2 * kTrainD + train_weights() + 2048 + 1024;
+constexpr int kTrainRed = kNL * (kTrainThreads / 32) * 16 * 4;  // column sums: [layer][warp][16]
+constexpr int kTrainSmem = 2 * kTrainX + (2 + kNHid) * kTrainH + 2 * kTrainD + train_weights() + kTrainRed + 1024;
 constexpr int kTrainCols = (kNHid + 1) * kHid + kOutPad + kOutPad + (kNHid - 1) * kHid + kInPad;  // tensor-memory columns
 // the shapes it is built for (default 17-64-64-8: 114 KB, 320 columns); others train by the kernel chain
 constexpr bool kTrainFused = kHid <= 64 && kTrainSmem <= 227 * 1024 && kTrainCols <= 512;
@@ -320,8 +328,10 @@ struct TrainArgs {
     const Scaling *sc;
     const bf16 *Wt[kNL], *Wn[kNL];
     const float *b[kNL];
-    float *part;   // [block][parameters] gradient sums
-    float *lpart;  // [block] loss sums
+    int split_tiles;  // row tiles of a split: 4 or 1
+    float *part;      // [split][parameters] weight gradients (the biases' places stay unused)
+    float *db[kNL];   // [tile] bias gradients, kTileRows apart (kOut: output layer)
+    float *lpart;     // [tile] loss sums
     int *err;
 };
 
@@ -360,7 +370,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_train(const __grid_constan
         Wt[l] = take(layer_k(l) * layer_n(l) * 2);
         Wn[l] = l > 0 ? take(layer_k(l) * layer_n(l) * 2) : nullptr;
     }
-    float *red = (float *)take(2048);  // [16 warps][16 columns], rows past the operands for M = 128 reads
+    float *red = (float *)take(kTrainRed);  // [layer][16 warps][16 columns], past the operands for M = 128 reads
     uint64_t *bar = (uint64_t *)take(1024);
     uint32_t *tslot = (uint32_t *)(bar + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -422,10 +432,15 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_train(const __grid_constan
 #pragma unroll
         for (int q = 0; q < kOut; q++) pt[q] = in && targets ? g.ts[idx * kOut + q] : 0.0f;
     };
-    fetch(blockIdx.x);
-    float bsum[kNHid], osum = 0.0f;  // this lane's running column sums: hidden biases; output biases and the loss
-#pragma unroll
-    for (int l = 0; l < kNHid; l++) bsum[l] = 0.0f;
+    // the block's tiles: those of the splits blockIdx.x, blockIdx.x + gridDim.x, ..., each split's in order
+    long long tile = blockIdx.x * (long long)g.split_tiles;
+    const int last = g.split_tiles - 1;
+    fetch(tile);
+    // this warp's sums of 16 columns of layer l (a bias's gradient; in the output layer also the loss)
+    auto put_sums = [&](int l, float v[16]) {
+        const float s = warp_column_sum16(v, lane);
+        if (!(lane & 1)) red[(l * (kTrainThreads / 32) + warp) * 16 + (lane >> 1)] = s;
+    };
     // 16 values of this row (columns 16 part ..) as operands of the next product and, transposed, of a gradient
     auto put = [&](const float v[16], bf16 *normal, bf16 *transposed) {
         if (normal) {
@@ -437,8 +452,10 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_train(const __grid_constan
         for (int q = 0; q < 16; q++) t[q * 8] = __float2bfloat16_rn(v[q]);
     };
     const bool hidden = part * 16 < kHid;  // this part has columns of a hidden layer
-    bool begun = false;
-    for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    bool begun = false;  // the accumulators hold earlier tiles of this split
+    while (tile < tiles) {
+        const bool ends = (tile & last) == last;
+        const long long next = tile + 1 + (ends ? (long long)(gridDim.x - 1) * g.split_tiles : 0);
         {   // standardised inputs; zero columns past kIn
             float x[8];
 #pragma unroll
@@ -451,7 +468,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_train(const __grid_constan
         float tgt[kOut];
 #pragma unroll
         for (int q = 0; q < kOut; q++) tgt[q] = targets ? pt[q] / g.sc->ysd[q] : 0.0f;
-        if (tile + gridDim.x < tiles) fetch(tile + gridDim.x);
+        if (next < tiles) fetch(next);
         // forward
 #pragma unroll
         for (int l = 0; l < kNHid; l++) {
@@ -484,7 +501,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_train(const __grid_constan
 #pragma unroll
             for (int q = 0; q < kOutPad; q++) t[q * 8] = __float2bfloat16_rn(v[q]);
             v[kOut] = l;
-            osum += warp_column_sum16(v, lane);
+            put_sums(kNHid, v);
         }
         // backward: deltas of layer l from those of layer l + 1, and the gradient of layer l + 1's weights
 #pragma unroll
@@ -505,51 +522,48 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_train(const __grid_constan
 #pragma unroll
                 for (int q = 0; q < 16; q++) v[q] *= smelu_d(z[q] + __ldg(g.b[l] + part * 16 + q));
                 put(v, l > 0 ? Hn : nullptr, Dt);
-                bsum[l] += warp_column_sum16(v, lane);
+                put_sums(l, v);
             }
         }
         products([&] { mma_run(gcol(0), Dt, kHid, Xt, kInPad, kTileRows / 16, begun); });
-        begun = true;
-    }
-    // this block's gradient in parameter order: the weight gradients are [n][k] for the hidden layers
-    // (lane n, column k) and [k][n] for the output layer
-    float *out = g.part + blockIdx.x * (long long)param_count();
-    const int n = rl;
+        // the tile's bias gradients and loss: column sums of the four warps that hold a column
+        if (tid < kNHid * kHid + kOut + 1) {
+            const int l = min(tid / kHid, kNHid), n = tid - l * kHid;
+            const int w0 = l == kNHid ? 4 * (kParts - 1) : (n >> 4) * 4;
+            const float *r = red + (l * (kTrainThreads / 32) + w0) * 16 + (n & 15);
+            const float v = r[0] + r[16] + r[32] + r[48];
+            if (l < kNHid) g.db[l][tile * kTileRows + n] = v;
+            else if (n < kOut) g.db[l][tile * kOut + n] = v;
+            else g.lpart[tile] = v;
+        }
+        // the split's weight gradients in parameter order: [n][k] for the hidden layers (lane n, column
+        // k) and [k][n] for the output layer
+        if (ends) {
+            float *out = g.part + (tile / g.split_tiles) * (long long)param_count();
+            const int n = rl;
 #pragma unroll
-    for (int l = 0; l < kNL; l++) {
-        const int cols = l == kNHid ? kOutPad : l == 0 ? kInPad : kHid;
-        if (part * 16 < cols) {
-            float v[16];
-            tmem_ld16(gcol(l) + part * 16 + lanes, v);
-            if (n < kHid) {
+            for (int l = 0; l < kNL; l++) {
+                const int cols = l == kNHid ? kOutPad : l == 0 ? kInPad : kHid;
+                if (part * 16 < cols) {
+                    float v[16];
+                    tmem_ld16(gcol(l) + part * 16 + lanes, v);
+                    if (n < kHid) {
 #pragma unroll
-                for (int q = 0; q < 16; q++) {
-                    const int k = part * 16 + q;
-                    if (l == kNHid) {
-                        if (k < kOut) out[n * kOut + k] = v[q];
-                    } else if (k < real_k(l)) {
-                        out[k * kHid + n] = v[q];
+                        for (int q = 0; q < 16; q++) {
+                            const int k = part * 16 + q;
+                            if (l == kNHid) {
+                                if (k < kOut) out[n * kOut + k] = v[q];
+                            } else if (k < real_k(l)) {
+                                out[k * kHid + n] = v[q];
+                            }
+                        }
                     }
                 }
+                out += real_k(l) * real_n(l) + real_n(l);
             }
         }
-        out += real_k(l) * real_n(l) + real_n(l);
-    }
-    // biases: column sums of the four warps that hold a column
-    out = g.part + blockIdx.x * (long long)param_count();
-#pragma unroll
-    for (int l = 0; l < kNL; l++) {
-        out += real_k(l) * real_n(l);
-        __syncthreads();
-        if (!(lane & 1)) red[warp * 16 + (lane >> 1)] = l == kNHid ? osum : bsum[l < kNHid ? l : 0];
-        __syncthreads();
-        if (tid < (l == kNHid ? kOut + 1 : kHid)) {
-            const int w0 = l == kNHid ? 4 * (kParts - 1) : (tid >> 4) * 4, c = l == kNHid ? tid : tid & 15;
-            const float v = red[w0 * 16 + c] + red[(w0 + 1) * 16 + c] + red[(w0 + 2) * 16 + c] + red[(w0 + 3) * 16 + c];
-            if (l == kNHid && tid == kOut) g.lpart[blockIdx.x] = v;
-            else out[tid] = v;
-        }
-        out += real_n(l);
+        begun = !ends;
+        tile = next;
     }
     if (bad) atomicOr(g.err, NN_ERR_WAIT);
     tc_fence_before();
@@ -564,7 +578,7 @@ struct AdamArgs {
     float *W[kNL], *b[kNL], *mW[kNL], *vW[kNL], *mb[kNL], *vb[kNL];
     const float *dw[kNL];  // weight-gradient partials
     const float *db[kNL];  // bias-gradient partials
-    const float *part;     // or (not null) `splits` gradients in parameter order
+    const float *part;     // or (not null) weight-gradient partials in parameter order
     bf16 *Wt[kNL], *Wn[kNL], *Bt[kNHid];
     int splits, tiles;
     float lr, beta1, beta2, eps, c1, c2;  // c1 = 1 - beta1^t, c2 = 1 - beta2^t
@@ -574,11 +588,12 @@ struct AdamArgs {
 
 __host__ __device__ constexpr long long layer_params(int l) { return (long long)real_k(l) * real_n(l) + real_n(l); }
 
-// kAdamGroup threads per real parameter add its gradient partials (their loads coalesce over the 32
-// parameters of a block); the first of them does the Adam step on the FP32 master and writes the BF16
-// copies in both operand layouts.  One thread per parameter took 41 us for 128 splits: a serial chain
-// of loads on 23 blocks.
-constexpr int kAdamGroup = 8, kAdamParams = 32;
+// kAdamGroup threads per real parameter load its gradient partials (kAdamStage at a time, coalesced over
+// the 32 parameters of a block); the first of them adds them in order, does the Adam step on the FP32
+// master and writes the BF16 copies in both operand layouts.  Bound by the 512 ordered additions of a
+// bias at 65536 rows: 8 us (23 with the next stage's loads behind the additions instead of before them).
+// One thread per parameter that loaded its partials itself took 41 us: a serial chain of loads on 23 blocks.
+constexpr int kAdamGroup = 8, kAdamParams = 32, kAdamStage = 128;
 __global__ void __launch_bounds__(kAdamGroup * kAdamParams) k_adam(AdamArgs a) {
     const int col = threadIdx.x % kAdamParams, grp = threadIdx.x / kAdamParams;
     long long t = blockIdx.x * (long long)kAdamParams + col;
@@ -621,25 +636,44 @@ __global__ void __launch_bounds__(kAdamGroup * kAdamParams) k_adam(AdamArgs a) {
     } else {
         n = (int)(t - (long long)kr * nr);
     }
-    if (have) {
-        if (a.part) {
-            for (int s = grp; s < a.splits; s += kAdamGroup) g += a.part[(long long)s * param_count() + off + t];
-        } else if (is_w) {
-            // the weight-gradient product is [n][k] for the hidden layers and [k][n] for the output layer
-            for (int s = grp; s < a.splits; s += kAdamGroup)
-                g += (l < kNHid) ? a.dw[l][((long long)s * kTileRows + n) * dw_cols(l) + k]
-                                 : a.dw[l][((long long)s * kTileRows + k) * N + n];
-        } else {
-            const int stride = (l < kNHid) ? kTileRows : kOut;
-            for (int s = grp; s < a.tiles; s += kAdamGroup) g += a.db[l][(long long)s * stride + n];
-        }
+    // this parameter's partials: the weight-gradient product of the chain is [n][k] for the hidden layers
+    // and [k][n] for the output layer
+    const float *src;
+    long long step;
+    if (!is_w) {
+        src = a.db[l] + n;
+        step = l < kNHid ? kTileRows : kOut;
+    } else if (a.part) {
+        src = a.part + off + t;
+        step = param_count();
+    } else {
+        src = a.dw[l] + (l < kNHid ? n * dw_cols(l) + k : k * N + n);
+        step = kTileRows * (l < kNHid ? dw_cols(l) : N);
     }
-    __shared__ float sums[kAdamGroup][kAdamParams];
-    sums[grp][col] = g;
-    __syncthreads();
-    if (grp || !have) return;
+    const int count = !have ? 0 : is_w ? a.splits : a.tiles;
+    const int most = __syncthreads_or(have && !is_w) ? a.tiles : a.splits;  // a batch has no more splits than tiles
+    __shared__ float stage[kAdamStage][kAdamParams];
+    float in[kAdamStage / kAdamGroup];  // the stage after the one that is added: in flight meanwhile
+    auto load = [&](int s0) {
 #pragma unroll
-    for (int q = 1; q < kAdamGroup; q++) g += sums[q][col];
+        for (int q = 0; q < kAdamStage / kAdamGroup; q++) {
+            const int s = s0 + grp + q * kAdamGroup;
+            in[q] = s < count ? src[s * step] : 0.0f;  // past the end a zero: it changes no sum that began at +0
+        }
+    };
+    load(0);
+    for (int s0 = 0; s0 < most; s0 += kAdamStage) {
+#pragma unroll
+        for (int q = 0; q < kAdamStage / kAdamGroup; q++) stage[grp + q * kAdamGroup][col] = in[q];
+        __syncthreads();
+        load(s0 + kAdamStage);
+        if (grp == 0) {
+#pragma unroll 32
+            for (int s = 0; s < kAdamStage; s++) g += stage[s][col];
+        }
+        __syncthreads();
+    }
+    if (grp || !have) return;
     if (a.gout) a.gout[off + t] = g;
     if (!a.apply) return;
     float *p = is_w ? &a.W[l][k * N + n] : &a.b[l][n];
@@ -736,8 +770,8 @@ struct dg_nn {
     bf16 *Xn = nullptr, *Xt = nullptr, *Hn[kNHid] = {}, *Ht[kNHid] = {}, *Dn[2] = {}, *Dt[2] = {}, *D3n = nullptr,
          *D3t = nullptr;
     float *Tb = nullptr, *Y = nullptr, *G[kNHid] = {}, *dw[kNL] = {}, *db[kNL] = {}, *lpart = nullptr, *gout = nullptr;
-    float *part = nullptr;       // per-block gradients of the one-kernel pass (param_count() each) ...
-    long long lparts = 0;        // ... and the loss sums the last pass left in lpart
+    float *part = nullptr;       // weight gradients of the one-kernel pass by split (param_count() each)
+    long long scap = 0;          // splits that the gradient scratch holds
     long long step = 0;
     unsigned long long seed = 1;
     float beta1 = 0.9f, beta2 = 0.999f, eps = 1e-8f;
@@ -797,36 +831,42 @@ int scratch_alloc(dg_nn *n, void **p, size_t bytes) {
 }
 template <typename X> int scratch_t(dg_nn *n, X **p, size_t count) { return scratch_alloc(n, (void **)p, count * sizeof(X)); }
 
-// batch work arrays for `rows` rows (reallocated when a larger batch comes)
+// rows of one weight-gradient partial: 512 where they divide the batch, else one row tile
+long long split_rows(long long rows) { return rows % 512 == 0 ? 512 : kTileRows; }
+
+// batch work arrays for `rows` rows (reallocated when a larger batch, or one of more splits, comes)
 int ensure_batch(dg_nn *n, long long rows) {
-    if (rows <= n->bcap) return 0;
+    const long long R = std::max(rows, n->bcap), tiles = R / kTileRows;
+    const long long splits = std::max(rows / split_rows(rows), n->scap);
+    if (R <= n->bcap && splits <= n->scap) return 0;
     NN_CUDA(cudaStreamSynchronize(n->stream));
     for (void *p : n->scratch) cudaFree(p);
     n->scratch.clear();
-    n->bcap = 0;
+    n->bcap = n->scap = 0;
     int rc;
-    const long long R = rows, tiles = R / kTileRows;
-    const long long splits = R / ((R % 512 == 0) ? 512 : 128);
     if ((rc = scratch_t(n, &n->Xn, R * kInPad)) || (rc = scratch_t(n, &n->Xt, R * kInPad)) ||
         (rc = scratch_t(n, &n->Tb, R * kOut)) || (rc = scratch_t(n, &n->Y, R * kOut)) ||
         (rc = scratch_t(n, &n->D3n, R * kOutPad)) || (rc = scratch_t(n, &n->D3t, R * kOutPad)) ||
         (rc = scratch_t(n, &n->lpart, tiles)) || (rc = scratch_t(n, &n->gout, dg_nn_param_count())))
         return rc;
-    if (kTrainFused && (rc = scratch_t(n, &n->part, std::min<long long>(tiles, kTrainBlocks) * param_count()))) return rc;
+    for (int l = 0; l < kNL; l++)
+        if ((rc = scratch_t(n, &n->db[l], tiles * kTileRows))) return rc;
+    if (kTrainFused && (rc = scratch_t(n, &n->part, splits * param_count()))) return rc;
     for (int l = 0; l < kNHid; l++)
         if ((rc = scratch_t(n, &n->Hn[l], R * kHid)) || (rc = scratch_t(n, &n->Ht[l], R * kHidT)) ||
             (rc = scratch_t(n, &n->G[l], R * kHid)))
             return rc;
     if (kTrainFused) {  // the kernel chain's gradient operands are not used
-        n->bcap = rows;
+        n->bcap = R;
+        n->scap = splits;
         return 0;
     }
     for (int q = 0; q < 2; q++)
         if ((rc = scratch_t(n, &n->Dn[q], R * kHid)) || (rc = scratch_t(n, &n->Dt[q], R * kHidT))) return rc;
     for (int l = 0; l < kNL; l++)
-        if ((rc = scratch_t(n, &n->dw[l], splits * kTileRows * kHidT)) || (rc = scratch_t(n, &n->db[l], tiles * kTileRows)))
-            return rc;
-    n->bcap = rows;
+        if ((rc = scratch_t(n, &n->dw[l], splits * kTileRows * kHidT))) return rc;
+    n->bcap = R;
+    n->scap = splits;
     return 0;
 }
 
@@ -871,7 +911,7 @@ int forward(dg_nn *n, long long rows) {
 template <int = 0>
 int backward(dg_nn *n, long long rows, long long valid) {
     const long long tiles = rows / kTileRows;
-    const int csplit = (rows % 512 == 0) ? 512 : 128;
+    const int csplit = (int)split_rows(rows);
     const long long splits = rows / csplit;
     k_loss<<<(unsigned)tiles, 128, 0, n->stream>>>(n->Y, n->Tb, rows, valid, n->D3n, n->D3t, n->lpart, n->db[kNHid]);
     NN_CUDA(cudaGetLastError());
@@ -904,9 +944,6 @@ int backward(dg_nn *n, long long rows, long long valid) {
     return 0;
 }
 
-// blocks of the one-kernel pass: one per SM (its tensor memory)
-int train_blocks(long long rows) { return (int)std::min<long long>(rows / kTileRows, kTrainBlocks); }
-
 int adam(dg_nn *n, long long rows, float lr, int apply, float *gout) {
     AdamArgs a{};
     for (int l = 0; l < kNL; l++) {
@@ -914,12 +951,9 @@ int adam(dg_nn *n, long long rows, float lr, int apply, float *gout) {
         a.vb[l] = n->vb[l]; a.dw[l] = n->dw[l]; a.db[l] = n->db[l]; a.Wt[l] = n->Wt[l]; a.Wn[l] = n->Wn[l];
         if (l < kNHid) a.Bt[l] = n->Bt[l];
     }
-    a.splits = (int)(rows / ((rows % 512 == 0) ? 512 : 128));
+    a.splits = (int)(rows / split_rows(rows));
     a.tiles = (int)(rows / kTileRows);
-    if (kTrainFused) {
-        a.part = n->part;
-        a.splits = train_blocks(rows);
-    }
+    if (kTrainFused) a.part = n->part;
     a.lr = lr; a.beta1 = n->beta1; a.beta2 = n->beta2; a.eps = n->eps;
     if (apply == 1) n->step++;
     const double t = (double)(n->step > 0 ? n->step : 1);
@@ -949,15 +983,17 @@ int gradient_pass(dg_nn *n, long long rows, int random) {
         g.seed = n->seed + 0x9E37ull * (unsigned long long)n->step;
         g.sc = n->d_sc;
         for (int l = 0; l < kNL; l++) { g.Wt[l] = n->Wt[l]; g.Wn[l] = n->Wn[l]; g.b[l] = n->b[l]; }
+        for (int l = 0; l < kNL; l++) g.db[l] = n->db[l];
+        g.split_tiles = (int)(split_rows(rows) / kTileRows);
         g.part = n->part; g.lpart = n->lpart; g.err = n->d_err;
-        n->lparts = train_blocks(rows);
         NN_CUDA(cudaFuncSetAttribute(k_train, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrainSmem));
-        k_train<<<(unsigned)n->lparts, kTrainThreads, kTrainSmem, n->stream>>>(g);
+        // a block per split, at most one per SM (its tensor memory)
+        const long long splits = rows / split_rows(rows);
+        k_train<<<(unsigned)std::min<long long>(splits, kTrainBlocks), kTrainThreads, kTrainSmem, n->stream>>>(g);
         NN_CUDA(cudaGetLastError());
         return 0;
     } else {
         int rc;
-        n->lparts = rows / kTileRows;
         if ((rc = gather(n, rows, random, 0)) || (rc = forward(n, rows))) return rc;
         return backward<>(n, rows, rows);
     }
@@ -1163,7 +1199,7 @@ int dg_nn_train(dg_nn *n, int steps, int batch, float lr, float *loss_out) {
         if ((rc = gradient_pass(n, batch, 1)) || (rc = adam(n, batch, lr, 1, nullptr))) return rc;
     }
     if (loss_out) {
-        std::vector<float> lp((size_t)n->lparts);
+        std::vector<float> lp((size_t)batch / kTileRows);
         NN_CUDA(cudaMemcpyAsync(lp.data(), n->lpart, lp.size() * sizeof(float), cudaMemcpyDeviceToHost, n->stream));
         if ((rc = nn_sync(n))) return rc;
         double l = 0.0;
@@ -1211,12 +1247,12 @@ int dg_nn_gradients(dg_nn *n, const float *x, const float *t, int batch, float *
         return rc;
     }
     NN_CUDA(cudaMemcpyAsync(n->gh, n->gout, (size_t)np * sizeof(float), cudaMemcpyDeviceToHost, n->stream));
-    NN_CUDA(cudaMemcpyAsync(n->gh + np, n->lpart, (size_t)n->lparts * sizeof(float), cudaMemcpyDeviceToHost, n->stream));
+    NN_CUDA(cudaMemcpyAsync(n->gh + np, n->lpart, (size_t)nl * sizeof(float), cudaMemcpyDeviceToHost, n->stream));
     if ((rc = nn_sync(n))) return rc;
     std::memcpy(grad, n->gh, (size_t)np * sizeof(float));
     if (loss) {
         double l = 0.0;
-        for (long long q = 0; q < n->lparts; q++) l += n->gh[np + q];
+        for (long long q = 0; q < nl; q++) l += n->gh[np + q];
         *loss = (float)(l / ((double)batch * kOut));
     }
     return DG_OK;
