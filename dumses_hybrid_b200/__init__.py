@@ -143,6 +143,7 @@ def load_library(path: str | pathlib.Path | None = None) -> ctypes.CDLL:
         "dg_nn_fit_envelope": (ctypes.c_int, [vp, ctypes.c_float]),
         "dg_nn_fit_scaling": (ctypes.c_int, [vp]),
         "dg_nn_set_gates": (ctypes.c_int, [vp, ctypes.c_float, ctypes.c_float]),
+        "dg_nn_wait_bound": (ctypes.c_int, [vp, ctypes.c_double]),
         "dg_attach_surrogate": (ctypes.c_int, [vp, vp]),
         "dg_wait_selftest": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, dp]),
         "dg_debug_oob_count": (ctypes.c_longlong, []),

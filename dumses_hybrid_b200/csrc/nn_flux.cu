@@ -333,6 +333,7 @@ struct TrainArgs {
     float *db[kNL];   // [tile] bias gradients, kTileRows apart (kOut: output layer)
     float *lpart;     // [tile] loss sums
     int *err;
+    unsigned long long wait_ns;  // bound of a wait
 };
 
 // column sums over a warp: lane L returns the sum over all lanes of v[L >> 1] (each exchange
@@ -358,6 +359,9 @@ __device__ __forceinline__ void mma_run(uint32_t d, const void *a, int arows, co
                  idesc_bf16(kTileRows, n), s > 0 || acc);
 }
 
+// the second wait of a block whose wait ran out: out of line, it is 1% of the kernel's time otherwise
+__device__ __noinline__ void drain(uint64_t *bar, unsigned parity) { mbar_wait(bar, parity); }
+
 __global__ void __launch_bounds__(kTrainThreads, 1) k_train(const __grid_constant__ TrainArgs g) {
     extern __shared__ __align__(1024) unsigned char sm[];
     unsigned char *at = sm;
@@ -373,11 +377,13 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_train(const __grid_constan
     float *red = (float *)take(kTrainRed);  // [layer][16 warps][16 columns], past the operands for M = 128 reads
     uint64_t *bar = (uint64_t *)take(1024);
     uint32_t *tslot = (uint32_t *)(bar + 1);
+    int *stop = (int *)(bar + 2);  // [phase]: a wait ran out in the product before one of this phase
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rl = tid & (kTileRows - 1), part = tid / kTileRows;  // row of the tile, and 16 columns of a layer
     if (tid == 0) {
         mbar_init(bar, 1);
         mbar_fence_init();
+        stop[0] = stop[1] = 0;
     }
     if (warp == 0) tmem_alloc(tslot, 512);
     for (int l = 0; l < kNL; l++) {
@@ -397,20 +403,29 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_train(const __grid_constan
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
 
     unsigned phase = 0;
-    bool bad = false;
-    // make this tile's operands visible, have thread 0 issue the products, and wait for them
+    bool late = false;  // a wait of this thread ran out
+    // Make this tile's operands visible, have thread 0 issue the products, and wait for them.  Once a wait
+    // has run out in any thread, all of them get false here and nothing more is issued; that thread waits a
+    // second time first, so that no product outlives the operands, the tensor memory or the block.  The
+    // word they read was written before the barrier and is not written again before the next one.
     auto products = [&](auto issue) {
         fence_async_smem();
         tc_fence_before();
         __syncthreads();
+        if (*(volatile int *)(stop + phase)) return false;
         if (tid == 0) {
             tc_fence_after();
             issue();
             mma_commit(bar);
         }
-        if (!bad) bad = !mbar_wait(bar, phase);
+        if (!mbar_wait(bar, phase, g.wait_ns)) {
+            late = true;
+            stop[phase ^ 1] = 1;
+            drain(bar, phase);
+        }
         phase ^= 1;
         tc_fence_after();
+        return true;
     };
     const long long tiles = g.rows / kTileRows;
     // this thread's 8 of the 32 padded input columns; the last part has only padding and takes the targets
@@ -453,7 +468,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_train(const __grid_constan
     };
     const bool hidden = part * 16 < kHid;  // this part has columns of a hidden layer
     bool begun = false;  // the accumulators hold earlier tiles of this split
-    while (tile < tiles) {
+    auto pass = [&]() {  // this tile; false, to all threads alike, when a wait ran out
         const bool ends = (tile & last) == last;
         const long long next = tile + 1 + (ends ? (long long)(gridDim.x - 1) * g.split_tiles : 0);
         {   // standardised inputs; zero columns past kIn
@@ -472,7 +487,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_train(const __grid_constan
         // forward
 #pragma unroll
         for (int l = 0; l < kNHid; l++) {
-            products([&] { mma_run(zcol + l * kHid, l == 0 ? Xn : Hn, kTileRows, Wt[l], kHid, layer_k(l) / 16, 0); });
+            if (!products([&] { mma_run(zcol + l * kHid, l == 0 ? Xn : Hn, kTileRows, Wt[l], kHid, layer_k(l) / 16, 0); })) return false;
             if (hidden) {
                 float v[16];
                 tmem_ld16(zcol + l * kHid + part * 16 + lanes, v);
@@ -481,7 +496,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_train(const __grid_constan
                 put(v, Hn, Ht[l]);
             }
         }
-        products([&] { mma_run(ocol, Hn, kTileRows, Wt[kNHid], kOutPad, kHid / 16, 0); });
+        if (!products([&] { mma_run(ocol, Hn, kTileRows, Wt[kNHid], kOutPad, kHid / 16, 0); })) return false;
         if (targets) {  // mean-squared-error gradient of the outputs, sums of the loss and the output biases
             float v[16];
             tmem_ld16(ocol + lanes, v);
@@ -506,7 +521,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_train(const __grid_constan
         // backward: deltas of layer l from those of layer l + 1, and the gradient of layer l + 1's weights
 #pragma unroll
         for (int l = kNHid - 1; l >= 0; l--) {
-            products([&] {
+            if (!products([&] {
                 if (l == kNHid - 1) {
                     mma_run(acol, On, kTileRows, Wn[l + 1], kHid, kOutPad / 16, 0);
                     mma_run(gcol(l + 1), Ht[l], kHid, Ot, kOutPad, kTileRows / 16, begun);
@@ -514,7 +529,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_train(const __grid_constan
                     mma_run(acol, Hn, kTileRows, Wn[l + 1], kHid, kHid / 16, 0);
                     mma_run(gcol(l + 1), Dt, kHid, Ht[l], kHid, kTileRows / 16, begun);
                 }
-            });
+            })) return false;
             if (hidden) {
                 float v[16], z[16];
                 tmem_ld16(acol + part * 16 + lanes, v);
@@ -525,7 +540,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_train(const __grid_constan
                 put_sums(l, v);
             }
         }
-        products([&] { mma_run(gcol(0), Dt, kHid, Xt, kInPad, kTileRows / 16, begun); });
+        if (!products([&] { mma_run(gcol(0), Dt, kHid, Xt, kInPad, kTileRows / 16, begun); })) return false;
         // the tile's bias gradients and loss: column sums of the four warps that hold a column
         if (tid < kNHid * kHid + kOut + 1) {
             const int l = min(tid / kHid, kNHid), n = tid - l * kHid;
@@ -564,8 +579,10 @@ __global__ void __launch_bounds__(kTrainThreads, 1) k_train(const __grid_constan
         }
         begun = !ends;
         tile = next;
-    }
-    if (bad) atomicOr(g.err, NN_ERR_WAIT);
+        return true;
+    };
+    while (tile < tiles && pass()) {}
+    if (late) atomicOr(g.err, NN_ERR_WAIT);
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {
@@ -584,6 +601,7 @@ struct AdamArgs {
     float lr, beta1, beta2, eps, c1, c2;  // c1 = 1 - beta1^t, c2 = 1 - beta2^t
     int apply;                             // 1: Adam step; 0: only reduce the gradient; 2: only pack BF16 copies
     float *gout;                           // reduced gradients in parameter order (or null)
+    const int *err;                        // the gradient pass's error word: no step from an invalid gradient
 };
 
 __host__ __device__ constexpr long long layer_params(int l) { return (long long)real_k(l) * real_n(l) + real_n(l); }
@@ -605,6 +623,7 @@ __global__ void __launch_bounds__(kAdamGroup * kAdamParams) k_adam(AdamArgs a) {
     for (int q = 0; q < l; q++) off += layer_params(q);
     const int K = layer_k(l), N = layer_n(l), kr = real_k(l), nr = real_n(l);
     const bool is_w = t < (long long)kr * nr;
+    if (a.apply == 1 && *a.err) return;
     float g = 0.0f;
     int k = 0, n = 0;
     // the face kernel's bias operand of hidden layer l < kNHid (its columns 2.. stay zero)
@@ -774,6 +793,7 @@ struct dg_nn {
     long long scap = 0;          // splits that the gradient scratch holds
     long long step = 0;
     unsigned long long seed = 1;
+    unsigned long long wait_ns = kWaitNs;  // bound of a wait in the one-kernel pass
     float beta1 = 0.9f, beta2 = 0.999f, eps = 1e-8f;
     Gates gates{};
     Scaling sc{};              // host copy of the standardisation
@@ -961,6 +981,7 @@ int adam(dg_nn *n, long long rows, float lr, int apply, float *gout) {
     a.c2 = (float)(1.0 - std::pow((double)n->beta2, t));
     a.apply = apply;
     a.gout = gout;
+    a.err = n->d_err;
     const long long np = dg_nn_param_count();
     k_adam<<<(unsigned)((np + kAdamParams - 1) / kAdamParams), kAdamGroup * kAdamParams, 0, n->stream>>>(a);
     NN_CUDA(cudaGetLastError());
@@ -985,7 +1006,7 @@ int gradient_pass(dg_nn *n, long long rows, int random) {
         for (int l = 0; l < kNL; l++) { g.Wt[l] = n->Wt[l]; g.Wn[l] = n->Wn[l]; g.b[l] = n->b[l]; }
         for (int l = 0; l < kNL; l++) g.db[l] = n->db[l];
         g.split_tiles = (int)(split_rows(rows) / kTileRows);
-        g.part = n->part; g.lpart = n->lpart; g.err = n->d_err;
+        g.part = n->part; g.lpart = n->lpart; g.err = n->d_err; g.wait_ns = n->wait_ns;
         NN_CUDA(cudaFuncSetAttribute(k_train, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrainSmem));
         // a block per split, at most one per SM (its tensor memory)
         const long long splits = rows / split_rows(rows);
@@ -1371,6 +1392,12 @@ int dg_nn_fit_scaling(dg_nn *n) {
     }
     NN_CUDA(cudaMemcpyAsync(n->d_sc, &n->sc, sizeof(Scaling), cudaMemcpyHostToDevice, n->stream));
     return nn_sync(n);
+}
+
+int dg_nn_wait_bound(dg_nn *n, double seconds) {
+    if (!n || !(seconds >= 0.0) || seconds > 60.0) return nn_fail(DG_ERR_ARG, "bad wait bound");
+    n->wait_ns = (unsigned long long)(seconds * 1e9);
+    return DG_OK;
 }
 
 int dg_nn_set_gates(dg_nn *n, float jump, float compress) {

@@ -43,8 +43,9 @@ __device__ __forceinline__ unsigned long long global_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-// poll the phase with the given parity; false when kWaitNs ran out first
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity) {
+// poll the phase with the given parity; false when the bound ran out first (0: without a poll)
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, unsigned long long bound_ns = kWaitNs) {
+    if (bound_ns == 0) return false;
     const uint32_t a = smem_addr(bar);
     const unsigned long long t0 = global_ns();
     for (unsigned n = 1;; n++) {
@@ -57,7 +58,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity) {
             : "r"(a), "r"(parity)
             : "memory");
         if (done) return true;
-        if ((n & 255) == 0 && global_ns() - t0 > kWaitNs) return false;
+        if ((n & 255) == 0 && global_ns() - t0 > bound_ns) return false;
     }
 }
 

@@ -352,6 +352,11 @@ int  dg_nn_fit_envelope(dg_nn *nn, float margin);
  * the current samples; call before training (identity until then) */
 int  dg_nn_fit_scaling(dg_nn *nn);
 int  dg_nn_set_gates(dg_nn *nn, float jump, float compress);
+/* Bound of each device-side wait of dg_nn_train and dg_nn_gradients (networks up to 64 wide), 0 to 60
+ * seconds, 1 by default.  A pass whose wait runs out stops, leaves the parameters as they were and is
+ * reported as DG_ERR_STATE by this call and by the network's later ones.  With 0 every wait runs out at
+ * once (the products in flight are still waited for, up to a second): what the test of this path sets. */
+int  dg_nn_wait_bound(dg_nn *nn, double seconds);
 /* use `nn` (NULL: none) for the faces of an FP32 context made with surrogate = 1 */
 int  dg_attach_surrogate(dg_ctx *ctx, dg_nn *nn);
 /* faces seen by the surrogate and faces that fell back to HLLD since the last call */
