@@ -23,13 +23,21 @@ constexpr double kSmallc = 1.0e-10;  // commons.f90:49
 
 template <typename T> __host__ __device__ __forceinline__ T mn(T a, T b) { return a < b ? a : b; }
 template <typename T> __host__ __device__ __forceinline__ T mx(T a, T b) { return a > b ? a : b; }
-// x held at a floor; a NaN stays one.  FP32: one instruction instead of a compare and a select
-__device__ __forceinline__ double floored(double small, double x) { return mx(small, x); }
-__device__ __forceinline__ float floored(float small, float x) {
+// FP32 minimum and maximum in one instruction (a ternary is a compare and a select) that is a NaN where
+// either operand is one (fminf and fmaxf drop it): an invalid state spreads as it does in FP64
+__device__ __forceinline__ float mn_nan(float a, float b) {
     float r;
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(small), "f"(x));
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
     return r;
 }
+__device__ __forceinline__ float mx_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+// x held at a floor; a NaN stays one
+__device__ __forceinline__ double floored(double small, double x) { return mx(small, x); }
+__device__ __forceinline__ float floored(float small, float x) { return mx_nan(small, x); }
 __device__ __forceinline__ double sgn1(double x) { return copysign(1.0, x); }
 __device__ __forceinline__ float sgn1(float x) { return copysignf(1.0f, x); }
 __device__ __forceinline__ double fab(double x) { return fabs(x); }

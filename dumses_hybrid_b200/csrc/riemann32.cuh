@@ -248,8 +248,8 @@ __device__ __forceinline__ V2 hlld2d_2(const Corner2 &LL, const Corner2 &LR, con
     fast(LR, x1, y1, pLR);
     fast(RL, x2, y2, pRL);
     fast(RR, x3, y3, pRR);
-    auto mx4v = [](V2 a, V2 b, V2 c, V2 d) { return max2(max2(max2(a, b), c), d); };
-    auto mn4v = [](V2 a, V2 b, V2 c, V2 d) { return min2(min2(min2(a, b), c), d); };
+    auto mx4v = [](V2 a, V2 b, V2 c, V2 d) { return p2(mx4(a.x, b.x, c.x, d.x), mx4(a.y, b.y, c.y, d.y)); };
+    auto mn4v = [](V2 a, V2 b, V2 c, V2 d) { return p2(mn4(a.x, b.x, c.x, d.x), mn4(a.y, b.y, c.y, d.y)); };
     const V2 cfx = root2(mx4v(x0, x1, x2, x3)), cfy = root2(mx4v(y0, y1, y2, y3));
     const V2 SL = mn4v(LL.u, LR.u, RL.u, RR.u) - cfx, SR = mx4v(LL.u, LR.u, RL.u, RR.u) + cfx;
     const V2 SB = mn4v(LL.v, LR.v, RL.v, RR.v) - cfy, ST = mx4v(LL.v, LR.v, RL.v, RR.v) + cfy;

@@ -366,9 +366,8 @@ struct Corners {
 
 template <typename T> __device__ __forceinline__ T mn4(T a, T b, T c, T d) { return mn(mn(mn(a, b), c), d); }
 template <typename T> __device__ __forceinline__ T mx4(T a, T b, T c, T d) { return mx(mx(mx(a, b), c), d); }
-// FP32: one instruction per minimum or maximum (a ternary is a compare and a select)
-__device__ __forceinline__ float mn4(float a, float b, float c, float d) { return fminf(fminf(fminf(a, b), c), d); }
-__device__ __forceinline__ float mx4(float a, float b, float c, float d) { return fmaxf(fmaxf(fmaxf(a, b), c), d); }
+__device__ __forceinline__ float mn4(float a, float b, float c, float d) { return mn_nan(mn_nan(mn_nan(a, b), c), d); }
+__device__ __forceinline__ float mx4(float a, float b, float c, float d) { return mx_nan(mx_nan(mx_nan(a, b), c), d); }
 
 template <typename T>
 __device__ T llf2d(const Corners<T> &c, T dt, T gamma, T ciso, int iso) {

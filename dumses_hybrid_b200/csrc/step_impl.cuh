@@ -440,10 +440,11 @@ __device__ __forceinline__ T limit1(T st, T qm1, T q0, T qp1) {
     const T half = T(0.5);
     if constexpr (sizeof(T) == 4) {
         // FP32: min(st |dl|, st |dr|) = st min(|dl|, |dr|) and the centred difference needs no st; with
-        // one-instruction minima this is 11 instructions (33 limiters a cell: trace 1.23 -> 1.18 ms at 256^3)
+        // one-instruction minima this is 11 instructions (33 limiters a cell: trace 1.23 -> 1.18 ms at 256^3).
+        // A NaN in any of the three values makes dcen one, and so the slope
         const T dl = q0 - qm1, dr = qp1 - q0, dcen = half * (dl + dr);
         const T dlim = dl * dr <= T(0) ? T(0) : st * fminf(fabsf(dl), fabsf(dr));
-        return copysignf(fminf(dlim, fabsf(dcen)), dcen);
+        return copysignf(mn_nan(dlim, fabsf(dcen)), dcen);
     } else {
         const T dlft = st * (q0 - qm1);
         const T drgt = st * (qp1 - q0);
