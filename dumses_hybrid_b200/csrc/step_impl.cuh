@@ -797,14 +797,12 @@ constexpr int kRingQ = 4, kRingE = 2;
 // least time by that count over the waves of resident blocks: 10 to 16 planes on large grids (10, 16
 // and 29 take the same time at 256^3), fewer where marches that long leave most of the chip idle
 // (FP64, both parts, always 16 planes -> this rule: 32 x 64 x 32 cells 0.104 -> 0.039 ms, 64^3 0.117 ->
-// 0.073, 101 x 75 x 53 0.127 -> 0.092; FP32, 32 x 64 x 32 cells: 0.054 -> 0.021).  A column of more planes
-// than 65535 marches of one needs longer ones.
+// 0.073, 101 x 75 x 53 0.127 -> 0.092; FP32, 32 x 64 x 32 cells: 0.054 -> 0.021).
 constexpr double kTraceFill = 2.5;
 inline int trace_march(int tiles, int planes, int slots) {
-    const int shortest = (planes + 65534) / 65535;  // a launch has at most 65535 blocks along z
-    int best = shortest;
+    int best = 1;
     double least = 1e300;
-    for (int kz = shortest; kz <= 16 && kz <= planes; kz++) {
+    for (int kz = 1; kz <= 16 && kz <= planes; kz++) {
         const long long blocks = (long long)tiles * ((planes + kz - 1) / kz);
         const double cost = (double)((blocks + slots - 1) / slots) * (kz + kTraceFill);
         if (cost <= least) { least = cost; best = kz; }
