@@ -4,7 +4,8 @@
   with fractional multi-cell shifts (1-8 cells, fargo.f90:128-240 summing B over the
   traversed cells), through dg_fargo_update alone;
 - the MRI + FARGO shearing box at 64 x 128 x 32 with a slow sound speed, so that most
-  columns shift by one cell or more per step and every y line spans 9 FARGO segments;
+  columns shift by one cell or more per step and every y line spans 33 FARGO segments of 4 rows
+  (test_fargo_segments_gpu.py has the grids that take segments of 16);
 - the 3D Orszag-Tang vortex at 128^3 (many 32-cell trace-core blocks per row);
 - grids past 2^31 trace-core elements (64-bit indexing), checked by a property that does
   not depend on size: a periodic state tiled in y and z evolves into the tiled evolution
@@ -66,8 +67,8 @@ def test_fargo_fractional_multi_cell_shifts():
 
 
 def test_fargo_long_lines_and_shifts_above_the_segment():
-    # 8 x 64 columns: 65 y faces per line (5 segments of 16), shifts of 3-25 cells,
-    # larger than a segment
+    # 8 x 64 columns: 65 y faces per line (17 segments of 4), shifts of 3-25 cells,
+    # larger than a segment of either length
     p = Params(**{**fargo_params().__dict__, "ny": 64, "ymax": 1.0})
     dt = 0.55
     s = shifts(p, dt)
