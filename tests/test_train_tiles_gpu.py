@@ -1,5 +1,6 @@
-"""The fused gradient pass (k_train, csrc/nn_flux.cu) where its grid changes: a single row tile of 128, one
-tile per block (148 tiles), one block with a second tile, and a ragged third round.  Tolerance: the
+"""The fused gradient pass (k_train, csrc/nn_flux.cu) where its grid changes: a single row tile of 128, 37
+blocks of four tiles (148 tiles, a multiple of 512 rows), 149 splits of one tile on 148 blocks, and a ragged
+third round of them.  The order of its sums is held in test_train_sums_gpu.py.  Tolerance here: the
 2e-3 relative L2 per layer of the gradient tests (BF16 operands, FP32 sums); the loss to 1e-3."""
 import numpy as np
 import pytest
