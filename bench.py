@@ -542,8 +542,8 @@ def main() -> None:
                 except Exception:
                     pass
             return out
-        # the slot's time per step (the FP64 Riemann slot is six launches per step: faces and
-        # edges of each direction) against the step's algorithmic bytes of the 8 state variables
+        # the slot's time per step (the FP64 trace slot is two launches per step: cell fields, then
+        # face fields) against the step's algorithmic bytes of the 8 state variables
         slot_s = kernels[dom]["ms_total"] / args.steps / 1e3
         launches_per_step = kernels[dom]["launches"] / args.steps
         achieved = ALGO_BYTES_PER_ZONE * ncell / slot_s / 1e9

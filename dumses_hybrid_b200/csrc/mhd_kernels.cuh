@@ -17,7 +17,7 @@ struct Bufs {
     void *core;        // trace core over the core index space
     void *flx[3];      // face fluxes per direction, face-major records (flux_rec(ndim) values per face)
     void *emf[3];      // edge EMFs (x, y, z) over the face index space, already multiplied by dt
-    void *E[3];        // edge electric fields of the trace over the edge index space
+    void *E[3];        // edge electric fields of the trace over the edge index space (3D FP32: the harvest)
     double *femf[2];   // FARGO EMFs (x, z), FP64
     double *stage;     // FP64 staging planes for upload/download of the compensated state
     double *part;      // reduction partials
@@ -25,7 +25,7 @@ struct Bufs {
     Scalars *S;        // device scalars
     int nv;            // state variables: 8, or 9 with ndim = 2 (frozen right z-face)
     long long sv;      // cells per plane
-    int q_fresh;       // FP32 path: Q holds the primitive variables (without the rotation half-kick)
+    int q_fresh;       // Q holds the primitive variables (without the rotation half-kick)
                        // of U[cur], written by the last launch_dt with no state change since
     // learned face flux (FP32 path with surrogate = 1)
     const nn::NetView *net;         // attached network (host copy of its device view), null: HLLD everywhere

@@ -866,25 +866,23 @@ int ensure_batch(dg_nn *n, long long rows) {
     int rc;
     if ((rc = scratch_t(n, &n->Xn, R * kInPad)) || (rc = scratch_t(n, &n->Xt, R * kInPad)) ||
         (rc = scratch_t(n, &n->Tb, R * kOut)) || (rc = scratch_t(n, &n->Y, R * kOut)) ||
-        (rc = scratch_t(n, &n->D3n, R * kOutPad)) || (rc = scratch_t(n, &n->D3t, R * kOutPad)) ||
         (rc = scratch_t(n, &n->lpart, tiles)) || (rc = scratch_t(n, &n->gout, dg_nn_param_count())))
         return rc;
     for (int l = 0; l < kNL; l++)
         if ((rc = scratch_t(n, &n->db[l], tiles * kTileRows))) return rc;
-    if (kTrainFused && (rc = scratch_t(n, &n->part, splits * param_count()))) return rc;
     for (int l = 0; l < kNHid; l++)
         if ((rc = scratch_t(n, &n->Hn[l], R * kHid)) || (rc = scratch_t(n, &n->Ht[l], R * kHidT)) ||
             (rc = scratch_t(n, &n->G[l], R * kHid)))
             return rc;
-    if (kTrainFused) {  // the kernel chain's gradient operands are not used
-        n->bcap = R;
-        n->scap = splits;
-        return 0;
+    if constexpr (kTrainFused) {
+        if ((rc = scratch_t(n, &n->part, splits * param_count()))) return rc;
+    } else {  // the gradient operands of the kernel chain
+        if ((rc = scratch_t(n, &n->D3n, R * kOutPad)) || (rc = scratch_t(n, &n->D3t, R * kOutPad))) return rc;
+        for (int q = 0; q < 2; q++)
+            if ((rc = scratch_t(n, &n->Dn[q], R * kHid)) || (rc = scratch_t(n, &n->Dt[q], R * kHidT))) return rc;
+        for (int l = 0; l < kNL; l++)
+            if ((rc = scratch_t(n, &n->dw[l], splits * kTileRows * kHidT))) return rc;
     }
-    for (int q = 0; q < 2; q++)
-        if ((rc = scratch_t(n, &n->Dn[q], R * kHid)) || (rc = scratch_t(n, &n->Dt[q], R * kHidT))) return rc;
-    for (int l = 0; l < kNL; l++)
-        if ((rc = scratch_t(n, &n->dw[l], splits * kTileRows * kHidT))) return rc;
     n->bcap = R;
     n->scap = splits;
     return 0;

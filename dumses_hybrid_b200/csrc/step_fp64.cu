@@ -367,8 +367,8 @@ int launch_godunov(const Geo &G, const Bufs &B, int cur, cudaStream_t s) {
             const RiemannGrid rg = riemann64_grid(G);
             TIMED(KS_RIEMANN, s, (k_riemann64<<<rg.blocks, kThreads, 0, s>>>(G, rg.chunk, core, fx, fy, fz, ex, ey, ez, B.S)));
         } else {
-            TIMED(KS_RIEMANN, s, (k_faces3d<double, false><<<nb, kThreads, 0, s>>>(G, core, fx, fy, fz, B.S)));
-            TIMED(KS_RIEMANN, s, (k_edges3d<double, false><<<nb, kThreads, 0, s>>>(G, core, ex, ey, ez, B.S)));
+            TIMED(KS_RIEMANN, s, (k_faces3d<double><<<nb, kThreads, 0, s>>>(G, core, fx, fy, fz, B.S)));
+            TIMED(KS_RIEMANN, s, (k_edges3d<double><<<nb, kThreads, 0, s>>>(G, core, ex, ey, ez, B.S)));
             n++;
         }
         TIMED(KS_UPDATE, s, (k_update3d<<<nblocks(G.fsz, kThreads), kThreads, 0, s>>>(G, U.p, Un, fx, fy, fz, ex, ey, ez, B.S)));

@@ -10,16 +10,18 @@
 //
 // Pipeline of one step (the call order of src/dumses.f90:82-120):
 //   k_prim_dt     compute_dt  (physics.f90:18-132)      primitive(0) into Q + CFL min-reduction
-//   k_prim        primitive   (scheme.f90:20-91)        Q on the ghosted grid
-//   k_efield      edge E of trace3d/trace2d (scheme.f90:1194-1239, 856-872), once per edge
+//   k_prim        primitive   (scheme.f90:20-91)        Q on the ghosted grid, where no CFL pass left it
 //   k_trace       slope + trace3d/trace2d (scheme.f90:253-656, 807-1711), with primitive(dt)'s half-kick
+//                 and the edge E (scheme.f90:1194-1239, 856-872)
 //                 -> per-cell "trace core": predicted cell state, half slopes,
 //                    predicted face B and its transverse half slopes; every
 //                    face and corner state of the reference is one add (and a
 //                    floor) away from these values.
 //   k_riemann     riemann_solver + riemann_solver_magnetic + compflux
-//                 (solver.f90:65-387, solver_magnetic.f90:55-235, scheme.f90:1716-1760)
-//                 one thread per cell: its three left faces and three lower edges.
+//                 (solver.f90:65-387, solver_magnetic.f90:55-235, scheme.f90:1716-1760):
+//                 the three left faces and three lower edges of every cell, all in one thread
+//                 (k_riemann3d; two cells, k_riemann32) or one kind of solve per block (k_riemann64,
+//                 k_riemann2d).
 //   k_update      update + constrained_transport (scheme.f90:1764-1993), with the
 //                 shearing-box averaging of the boundary mass flux and emfy
 //                 (shearingbox.f90:207-390) applied on the fly.
@@ -263,12 +265,12 @@ __device__ __forceinline__ void finish_dt(const Geo &G, Scalars *S, unsigned lon
     set_shear(G, S);
 }
 
-// primitive variables of one cell in FP64 (scheme.f90:44-86); the right faces are the
-// neighbour's left faces (the frozen right z-face when ndim = 2)
+// primitive variables of one cell in FP64 (scheme.f90:44-77, without the rotation half-kick, which
+// needs dt: kick); the right faces are the neighbour's left faces (the frozen right z-face when ndim = 2)
 // (M: IeeeMath, or FastMath whose caller tests m.bad())
 template <class Store, class M>
 __device__ __forceinline__ void prim_cell(const Geo &G, const Store &U, long long c, double q[8], M &m) {
-    const double one = 1.0, half = 0.5, two = 2.0, dt = 0.0;
+    const double one = 1.0, half = 0.5;
     const double d = U.getr(G, IR, c);
     const auto id = m.rec(d);
     q[IR] = mx(d, kSmallr);
@@ -290,12 +292,6 @@ __device__ __forceinline__ void prim_cell(const Geo &G, const Store &U, long lon
         double emag = half * (q[IA] * q[IA] + q[IB] * q[IB] + q[IC] * q[IC]);
         double eint = m.div(U.getr(G, IP, c) - emag, d, id) - eken;
         q[IP] = mx((G.gamma - one) * q[IR] * eint, smallp);
-    }
-    if (G.omega0 > 0.0) {
-        double dvx = two * G.omega0 * q[IV];
-        double dvy = -(half * G.omega0 * q[IU]);
-        q[IU] = q[IU] + dvx * dt * half;
-        q[IV] = q[IV] + dvy * dt * half;
     }
 }
 
@@ -598,17 +594,10 @@ __device__ __forceinline__ T face_slope(const QV<T> &a, int c, int dir, int i, i
     return limit1(s, a.bf(c, i - di, j - dj, k - dk), a.bf(c, i, j, k), a.bf(c, i + di, j + dj, k + dk));
 }
 
-// resident blocks of 128 threads per SM that the trace and Riemann kernels are compiled
-// for (register caps 128/80 for the trace, 128/64 for the Riemann kernel, FP64/FP32),
-// chosen by timing the variants at 256^3
-#ifndef DG_TRACE_MINB64
-#define DG_TRACE_MINB64 4
-#endif
+// resident blocks of 128 threads per SM that the untiled trace and the one-cell Riemann kernel
+// (both FP32 only) are compiled for (register caps 80 and 64), chosen by timing the variants at 256^3
 #ifndef DG_TRACE_MINB32
 #define DG_TRACE_MINB32 6
-#endif
-#ifndef DG_RIEMANN_MINB64
-#define DG_RIEMANN_MINB64 4
 #endif
 #ifndef DG_RIEMANN_MINB32
 #define DG_RIEMANN_MINB32 8
@@ -762,7 +751,7 @@ __device__ __forceinline__ void trace3_cell(const Sten &a, const Geo &G, int i, 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 ? DG_TRACE_MINB64 : DG_TRACE_MINB32))
+__global__ void __launch_bounds__(kThreads, DG_TRACE_MINB32)
 k_trace3d(Geo G, const T *__restrict__ Q, const T *__restrict__ Bf, const T *__restrict__ Exa,
           const T *__restrict__ Eya, const T *__restrict__ Eza, T *__restrict__ core, const Scalars *S) {
     long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -776,7 +765,7 @@ k_trace3d(Geo G, const T *__restrict__ Q, const T *__restrict__ Bf, const T *__r
 
 // ---------------------------------------------------------------------------
 // The 3D trace with its stencil staged in shared memory.  A block of kThreads threads owns a
-// tile of kTX x kTY cells in (x, y) and marches along z through kTZ planes of the core index
+// tile of kTX x kTY cells in (x, y) and marches along z through kz planes (trace_march) of the core index
 // space.  Shared memory holds a ring of kRingQ z planes (k-1, k, k+1 and the one being
 // fetched) of the tile plus a one-cell halo in x and y, with the primitive variables and
 // left-face field components the part reads, and a ring of kRingE planes of the trace's edge
@@ -785,7 +774,7 @@ k_trace3d(Geo G, const T *__restrict__ Q, const T *__restrict__ Bf, const T *__r
 // alignment rule applies to the ghosted rows); cell plane k+2 is fetched while plane k is
 // computed.  Each stencil read is a shared-memory load at a fixed offset from the thread's
 // cell.  The parts (kPart as in trace3_cell) stage only what they read: part 1 the 8
-// primitives (its four face-B values come from global memory) and no edge fields, part 2 the
+// primitives (its face-B values go through slots of each thread's own) and no edge fields, part 2 the
 // velocities and the face-B components (for the edge fields), part 0 all of them.
 // ---------------------------------------------------------------------------
 constexpr int kTX = 32, kTY = kThreads / kTX;
@@ -1494,7 +1483,7 @@ __device__ T edge_emf(const Geo &G, const CoreView<T> &cv, long long cLL, long l
 }
 
 template <typename T, bool kHLLD>
-__global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 ? DG_RIEMANN_MINB64 : DG_RIEMANN_MINB32)) k_riemann3d(Geo G, const T *__restrict__ core, T *__restrict__ fx,
+__global__ void __launch_bounds__(kThreads, DG_RIEMANN_MINB32) k_riemann3d(Geo G, const T *__restrict__ core, T *__restrict__ fx,
                                                            T *__restrict__ fy, T *__restrict__ fz, T *__restrict__ ex,
                                                            T *__restrict__ ey, T *__restrict__ ez, const Scalars *S,
                                                            int faces) {
@@ -1562,25 +1551,18 @@ __device__ __forceinline__ double edge_emf_fast(const Geo &G, const double *core
     return edge_shear(G, c, emf, kDir, i, dtd);
 }
 
-// The same work split in two passes over the face index space: the face fluxes (1D solves)
+// FP64 with the other solvers: two passes over the face index space, the face fluxes (1D solves)
 // and the edge EMFs (2D solves), each compiled for its own register budget.  A thread
 // holds the live values of one kind of solve only, so more warps fit an SM; the trace core
-// is read twice (once per pass).  Every solve is the same function of the same core values
-// as in k_riemann3d, so the results are identical.
+// is read twice (once per pass).
 #ifndef DG_RFACE_MINB64
 #define DG_RFACE_MINB64 4
 #endif
 #ifndef DG_REDGE_MINB64
 #define DG_REDGE_MINB64 4
 #endif
-#ifndef DG_RFACE_MINB32
-#define DG_RFACE_MINB32 8
-#endif
-#ifndef DG_REDGE_MINB32
-#define DG_REDGE_MINB32 8
-#endif
-template <typename T, bool kHLLD>
-__global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 ? DG_RFACE_MINB64 : DG_RFACE_MINB32))
+template <typename T>
+__global__ void __launch_bounds__(kThreads, DG_RFACE_MINB64)
 k_faces3d(Geo G, const T *__restrict__ core, T *__restrict__ fx, T *__restrict__ fy, T *__restrict__ fz,
           const Scalars *S) {
     long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -1591,13 +1573,13 @@ k_faces3d(Geo G, const T *__restrict__ core, T *__restrict__ fx, T *__restrict__
     const double dt = S->dt;
     const CoreView<T> cv{core, kCore3};
     const long long c = G.cidx(i, j, k);
-    if (j <= G.ny && k <= G.nz) face_flux<T, kHLLD>(G, cv, G.cidx(i - 1, j, k), c, 0, i, dt, fx, t);
-    if (i <= G.nx && k <= G.nz) face_flux<T, kHLLD>(G, cv, G.cidx(i, j - 1, k), c, 1, i, dt, fy, t);
-    if (i <= G.nx && j <= G.ny) face_flux<T, kHLLD>(G, cv, G.cidx(i, j, k - 1), c, 2, i, dt, fz, t);
+    if (j <= G.ny && k <= G.nz) face_flux<T>(G, cv, G.cidx(i - 1, j, k), c, 0, i, dt, fx, t);
+    if (i <= G.nx && k <= G.nz) face_flux<T>(G, cv, G.cidx(i, j - 1, k), c, 1, i, dt, fy, t);
+    if (i <= G.nx && j <= G.ny) face_flux<T>(G, cv, G.cidx(i, j, k - 1), c, 2, i, dt, fz, t);
 }
 
-template <typename T, bool kHLLD>
-__global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 ? DG_REDGE_MINB64 : DG_REDGE_MINB32))
+template <typename T>
+__global__ void __launch_bounds__(kThreads, DG_REDGE_MINB64)
 k_edges3d(Geo G, const T *__restrict__ core, T *__restrict__ ex, T *__restrict__ ey, T *__restrict__ ez,
           const Scalars *S) {
     long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -1609,11 +1591,11 @@ k_edges3d(Geo G, const T *__restrict__ core, T *__restrict__ ex, T *__restrict__
     const CoreView<T> cv{core, kCore3};
     const long long c = G.cidx(i, j, k);
     if (k <= G.nz)
-        ez[t] = edge_emf<T, kHLLD>(G, cv, G.cidx(i - 1, j - 1, k), G.cidx(i, j - 1, k), G.cidx(i - 1, j, k), c, 2, i, dt);
+        ez[t] = edge_emf<T>(G, cv, G.cidx(i - 1, j - 1, k), G.cidx(i, j - 1, k), G.cidx(i - 1, j, k), c, 2, i, dt);
     if (j <= G.ny)
-        ey[t] = edge_emf<T, kHLLD>(G, cv, G.cidx(i - 1, j, k - 1), G.cidx(i - 1, j, k), G.cidx(i, j, k - 1), c, 1, i, dt);
+        ey[t] = edge_emf<T>(G, cv, G.cidx(i - 1, j, k - 1), G.cidx(i - 1, j, k), G.cidx(i, j, k - 1), c, 1, i, dt);
     if (i <= G.nx)
-        ex[t] = edge_emf<T, kHLLD>(G, cv, G.cidx(i, j - 1, k - 1), G.cidx(i, j, k - 1), G.cidx(i, j - 1, k), c, 0, i, dt);
+        ex[t] = edge_emf<T>(G, cv, G.cidx(i, j - 1, k - 1), G.cidx(i, j, k - 1), G.cidx(i, j - 1, k), c, 0, i, dt);
 }
 
 // ---------------------------------------------------------------------------
