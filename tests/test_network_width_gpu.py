@@ -1,8 +1,8 @@
-"""The network built 128 wide (-DDG_NN_WIDTH=128): its training pass does not fit one kernel and runs as the
-chain of one kernel per product (k_gemm, k_loss), which no other test reaches.  A library with that network
-code is linked here (the step's kernels in it stay 64 wide: only the network's own calls are made) and a child
-process runs the network's oracle tests on it, and the sums of a batch of more and smaller splits than an
-earlier, larger one."""
+"""The network built in other shapes (-DDG_NN_WIDTH, -DDG_NN_DEPTH).  128 wide its training pass does not fit
+one kernel and runs as the chain of one kernel per product (k_gemm, k_loss), which no other test reaches; the
+other shapes train in one kernel (k_train) with other operand sizes, column counts and numbers of links.  A
+library with that network code is linked here (the step's kernels in it keep the default shape: only the
+network's own calls are made) and a child process runs the network's tests on it."""
 import os
 import pathlib
 import subprocess
@@ -16,16 +16,14 @@ pytestmark = pytest.mark.gpu
 HERE = pathlib.Path(__file__).resolve().parent
 
 
-@pytest.fixture(scope="module")
-def wide_library(tmp_path_factory, built_library):
+def library(out, width, depth):
     from dumses_hybrid_b200 import build
-    out = tmp_path_factory.mktemp("wide")
     objs = [build.BUILD / (s + ".o") for s in [*build.CU_SOURCES, *build.CXX_SOURCES] if s != "nn_flux.cu"]
     if not all(o.exists() for o in objs):
         build.build(force=True)
-    obj, lib = out / "nn_flux.o", out / "libdumses_gpu_w128.so"
-    build._run([build._nvcc(), *build.NVCC_FLAGS, *build.CU_SOURCES["nn_flux.cu"], "-DDG_NN_WIDTH=128", "-c",
-                str(build.CSRC / "nn_flux.cu"), "-o", str(obj)], False)
+    obj, lib = out / "nn_flux.o", out / "libdumses_gpu_shape.so"
+    build._run([build._nvcc(), *build.NVCC_FLAGS, *build.CU_SOURCES["nn_flux.cu"], f"-DDG_NN_WIDTH={width}", f"-DDG_NN_DEPTH={depth}",
+                "-c", str(build.CSRC / "nn_flux.cu"), "-o", str(obj)], False)
     build._run([build._nvcc(), *build.ARCH, "-shared", "-cudart", "static", "-Xcompiler", "-fPIC", *map(str, objs),
                 str(obj), "-o", str(lib)], False)
     return lib
@@ -38,11 +36,18 @@ def child(lib, *args):
     return res.stdout
 
 
-def test_oracle_tests_of_the_network(wide_library):
-    names = ["test_forward_matches_oracle", "test_gradients_match_oracle", "test_adam_step_matches_oracle"]
-    out = child(wide_library, "-m", "pytest", "-q", "-p", "no:cacheprovider",
-                *[f"tests/test_nn_gpu.py::{n}" for n in names], "tests/test_train_tiles_gpu.py")
+ORACLE = ["tests/test_nn_gpu.py::" + n for n in ("test_forward_matches_oracle", "test_gradients_match_oracle",
+                                                 "test_adam_step_matches_oracle")] + ["tests/test_train_tiles_gpu.py"]
+
+
+def run_tests(lib, *tests):
+    out = child(lib, "-m", "pytest", "-q", "-p", "no:cacheprovider", *tests)
     assert " passed" in out and "skipped" not in out, out
+
+
+@pytest.mark.parametrize("width,depth", [(32, 2), (64, 1), (64, 3)])
+def test_one_kernel_shapes(tmp_path, built_library, width, depth):
+    run_tests(library(tmp_path, width, depth), *ORACLE, "tests/test_train_sums_gpu.py", "tests/test_train_wait_gpu.py")
 
 
 def sums():
@@ -71,6 +76,8 @@ def sums():
     print("sums held")
 
 
-def test_order_of_the_sums(wide_library):
-    assert "sums held" in child(wide_library, "-c", f"import sys; sys.path[:0] = ['.', {str(HERE)!r}]; "
+def test_kernel_chain(tmp_path, built_library):
+    lib = library(tmp_path, 128, 2)
+    run_tests(lib, *ORACLE)
+    assert "sums held" in child(lib, "-c", f"import sys; sys.path[:0] = ['.', {str(HERE)!r}]; "
                                 "import test_network_width_gpu as t; t.sums()")
